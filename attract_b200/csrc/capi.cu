@@ -7,7 +7,7 @@
 
 namespace att {
 cudaError_t launch_score(const KParams& p, int mode, int S, int K, int blocks, int threads, cudaStream_t st);
-cudaError_t occupancy_blocks(int mode, int S, int K, int threads, int rec_slot, int* blocks_per_sm);
+cudaError_t occupancy_blocks(int mode, int S, int K, int threads, int rec_slot, bool one_grid, int* blocks_per_sm);
 cudaError_t kernel_status(int* out, int clear, cudaStream_t st);
 cudaError_t kernel_debug_info(unsigned long long* out3, int clear, cudaStream_t st);
 int beads_per_lane(int S, int max_beads);
@@ -252,8 +252,8 @@ extern "C" int att_energrad(const AttGrid* grids, int n_grids, const AttLigands*
   return ATT_OK;
 }
 
-static int persistent_blocks(int mode, int S, int K, int threads, int rec_slot, const AttLaunchCfg* launch, int n_tiles,
-                             int* blocks) {
+static int persistent_blocks(int mode, int S, int K, int threads, int rec_slot, bool one_grid,
+                             const AttLaunchCfg* launch, int n_tiles, int* blocks) {
   if (launch && launch->blocks > 0) {
     *blocks = launch->blocks;
     return ATT_OK;
@@ -261,7 +261,7 @@ static int persistent_blocks(int mode, int S, int K, int threads, int rec_slot, 
   int dev = 0, sms = 0, per = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = occupancy_blocks(mode, S, K, threads, rec_slot, &per);
+  if (e == cudaSuccess) e = occupancy_blocks(mode, S, K, threads, rec_slot, one_grid, &per);
   if (e != cudaSuccess) return cuda_fail(e, "occupancy query");
   if (per < 1) per = 1;
   const int wpb = threads / 32;
@@ -308,12 +308,11 @@ extern "C" int att_minimise(const AttGrid* grids, int n_grids, const AttLigands*
   p.step0 = cfg->step0;
   if (n_tiles == 0) return ATT_OK;
   int blocks = 0;
-  rc = persistent_blocks(MODE_MIN, S, K, threads, p.rec_slot, launch, n_tiles, &blocks);
+  rc = persistent_blocks(MODE_MIN, S, K, threads, p.rec_slot,
+                         n_grids == 1 || p.grad_mode == ATT_GRAD_ANALYTIC, launch, n_tiles, &blocks);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMemsetAsync(work_counter_dev, 0, sizeof(int), st);
-  if (e != cudaSuccess) return cuda_fail(e, "att_minimise counter reset");
-  e = launch_score(p, MODE_MIN, S, K, blocks, threads, st);
+  cudaError_t e = launch_score(p, MODE_MIN, S, K, blocks, threads, st);
   if (e != cudaSuccess) return cuda_fail(e, "att_minimise launch");
   return ATT_OK;
 }
@@ -359,12 +358,11 @@ extern "C" int att_minimise_schema(const AttGrid* grids, int n_grids, const AttL
   }
   if (n_tiles == 0) return ATT_OK;
   int blocks = 0;
-  rc = persistent_blocks(MODE_QUAT, S, K, threads, p.rec_slot, launch, n_tiles, &blocks);
+  rc = persistent_blocks(MODE_QUAT, S, K, threads, p.rec_slot,
+                         n_grids == 1 || p.grad_mode == ATT_GRAD_ANALYTIC, launch, n_tiles, &blocks);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t e = cudaMemsetAsync(work_counter_dev, 0, sizeof(int), st);
-  if (e != cudaSuccess) return cuda_fail(e, "att_minimise_schema counter reset");
-  e = launch_score(p, MODE_QUAT, S, K, blocks, threads, st);
+  cudaError_t e = launch_score(p, MODE_QUAT, S, K, blocks, threads, st);
   if (e != cudaSuccess) return cuda_fail(e, "att_minimise_schema launch");
   return ATT_OK;
 }

@@ -1,0 +1,102 @@
+// Launches of the scoring kernels (score.cu): the kernel of a launch, its
+// shared memory and occupancy, and the kernels' error words.
+#include "score_parts.h"
+
+namespace att {
+
+static const void* kernel_of(int mode, int S, int K, bool one_grid) {
+  switch (mode) {
+    case MODE_EVAL:
+    case MODE_EVAL_MAT: return score_part_kernel<0>(mode, S, K, one_grid);
+    case MODE_MIN: return score_part_kernel<1>(mode, S, K, one_grid);
+    case MODE_BWD: return score_part_kernel<2>(mode, S, K, one_grid);
+    case MODE_QUAT: return score_part_kernel<3>(mode, S, K, one_grid);
+  }
+  return nullptr;
+}
+
+int beads_per_lane(int S, int max_beads) {
+  const int need = (max_beads + S - 1) / S;
+  int K = 1;
+  while (K < need) K <<= 1;
+  return K <= ATT_MAX_BEADS_PER_LANE ? K : ATT_MAX_BEADS_PER_LANE;  // larger ligands run in chunks
+}
+
+size_t score_smem_bytes(int K, int threads, int rec_slot) {
+  return warp_smem_bytes(K, rec_slot) * (size_t)(threads / 32);
+}
+
+// the shared memory of one block of `mode` (without bead arms unless the mode
+// accumulates dE/dmat)
+static size_t mode_smem_bytes(int mode, int K, int threads, int rec_slot) {
+  const bool arms = mode == MODE_EVAL_MAT || mode == MODE_QUAT;
+  return warp_smem_bytes(K, rec_slot, arms) * (size_t)(threads / 32);
+}
+
+static cudaError_t launch_one(const KParams& p, int mode, int S, int K, bool one_grid, int blocks, int threads,
+                              cudaStream_t st) {
+  const void* k = kernel_of(mode, S, K, one_grid);
+  if (k == nullptr) return cudaErrorInvalidValue;
+  const size_t smem = mode_smem_bytes(mode, K, threads, p.rec_slot);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && p.counter != nullptr) e = cudaMemsetAsync(p.counter, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  void* args[] = {const_cast<KParams*>(&p)};
+  return cudaLaunchKernel(k, dim3(blocks), dim3(threads), args, smem, st);
+}
+
+// One grid, or the reference gradient on several: one launch.  The analytic
+// gradient on several grids: one launch per grid over the same tiles, each
+// skipping the other grids' segments.  (The kernels over several grids hold the
+// reference mode only: the 32-lane, two-beads-per-lane evaluation compiled with
+// both modes reported a misaligned address in the analytic one, on lists that
+// continue in the CSR tail, where the bounds-checked build of the same source
+// found every index and alignment right.)
+cudaError_t launch_score(const KParams& p, int mode, int S, int K, int blocks, int threads, cudaStream_t st) {
+  if (p.n_grids == 1 || p.grad_mode == ATT_GRAD_REFERENCE)
+    return launch_one(p, mode, S, K, p.n_grids == 1, blocks, threads, st);
+  KParams q = p;
+  for (int g = 0; g < p.n_grids; ++g) {
+    q.grid[0] = p.grid[g];
+    q.grid_sel = g;
+    const cudaError_t e = launch_one(q, mode, S, K, true, blocks, threads, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// the bits of every part's error word
+cudaError_t kernel_status(int* out, int clear, cudaStream_t st) {
+  int w[SCORE_PARTS] = {0};
+  cudaError_t e = score_part_status<0>(&w[0], clear, st);
+  if (e == cudaSuccess) e = score_part_status<1>(&w[1], clear, st);
+  if (e == cudaSuccess) e = score_part_status<2>(&w[2], clear, st);
+  if (e == cudaSuccess) e = score_part_status<3>(&w[3], clear, st);
+  *out = 0;
+  for (int i = 0; i < SCORE_PARTS; ++i) *out |= w[i];
+  return e;
+}
+
+// the first failed check of the lowest part that has one
+cudaError_t kernel_debug_info(unsigned long long* out3, int clear, cudaStream_t st) {
+  unsigned long long w[SCORE_PARTS][3] = {};
+  cudaError_t e = score_part_debug<0>(w[0], clear, st);
+  if (e == cudaSuccess) e = score_part_debug<1>(w[1], clear, st);
+  if (e == cudaSuccess) e = score_part_debug<2>(w[2], clear, st);
+  if (e == cudaSuccess) e = score_part_debug<3>(w[3], clear, st);
+  int hit = 0;
+  while (hit < SCORE_PARTS - 1 && w[hit][0] == 0ull) ++hit;
+  for (int k = 0; k < 3; ++k) out3[k] = w[hit][k];
+  return e;
+}
+
+cudaError_t occupancy_blocks(int mode, int S, int K, int threads, int rec_slot, bool one_grid, int* blocks_per_sm) {
+  const void* k = kernel_of(mode, S, K, one_grid);
+  if (k == nullptr) return cudaErrorInvalidValue;
+  const size_t smem = mode_smem_bytes(mode, K, threads, rec_slot);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, threads, smem);
+}
+
+}  // namespace att

@@ -45,9 +45,36 @@
 
 #include <type_traits>
 
-#include "common.cuh"
+#include "score_parts.h"
+
+// This file is compiled once per part (a few modes each), so that the parts
+// build in parallel.
+#ifndef ATT_SCORE_PART
+#error "compile score.cu with -DATT_SCORE_PART=0 .. 3"
+#endif
 
 namespace att {
+
+// error word of this part's kernels (ATT_KERR_* bits); att_kernel_status()
+// reads and clears the words of all parts
+static __device__ int g_kernel_error = 0;
+
+// Debug builds (-DATT_BOUNDS_CHECK) check every computed index against its
+// buffer before the access, skip the access when it is out of range, and
+// record the first failure (check code, index, bound) for att_kernel_debug_info.
+static __device__ unsigned long long g_kernel_debug[3] = {0ull, 0ull, 0ull};
+#ifdef ATT_BOUNDS_CHECK
+static __device__ __noinline__ void bounds_report(int code, long long a, long long b) {
+  atomicOr(&g_kernel_error, ATT_KERR_BOUNDS);
+  if (atomicCAS(&g_kernel_debug[0], 0ull, (unsigned long long)code) == 0ull) {
+    g_kernel_debug[1] = (unsigned long long)a;
+    g_kernel_debug[2] = (unsigned long long)b;
+  }
+}
+#define ATT_CHECK(cond, code, a, b) ((cond) ? true : (bounds_report((code), (a), (b)), false))
+#else
+#define ATT_CHECK(cond, code, a, b) true
+#endif
 
 // ---------------------------------------------------------------------------
 // shared memory and copy helpers
@@ -62,6 +89,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // mbarrier: 3.8 % faster in the minimiser, per lane; 11 % faster for single
 // evaluations, spread over the warp.)
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
+  if (!ATT_CHECK(((dst | (uint32_t)(uintptr_t)src) & 15u) == 0u, 7, dst, (long long)(uintptr_t)src)) return;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ uint32_t lanemask_lt() {
@@ -98,7 +126,8 @@ __device__ __forceinline__ unsigned lds_u32(const void* p) {
 }
 
 __device__ __forceinline__ uint4 lds_u128(const void* p) {  // p 16-byte aligned
-  uint4 v;
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (!ATT_CHECK((smem_u32(p) & 15u) == 0u, 8, smem_u32(p), 0)) return v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "r"(smem_u32(p)) : "memory");
   return v;
@@ -108,55 +137,6 @@ __device__ __forceinline__ unsigned ldg_nc_u16(const uint16_t* p) {
   unsigned short v;
   asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
   return v;
-}
-
-// per-bead records shared by the team
-struct __align__(16) BeadPos {  // moved bead; w = ligand type (int bits)
-  float x, y, z;
-  int lt;
-};
-struct __align__(16) BeadArm {  // lever arm for the torque (Q x) or ligand-frame x (dE/dmat)
-  float x, y, z, pad;
-};
-
-// device-wide error word of the scoring kernels (ATT_KERR_* bits), read and
-// cleared by att_kernel_status()
-__device__ int g_kernel_error = 0;
-
-// Debug builds (-DATT_BOUNDS_CHECK) check every computed index against its
-// buffer before the access, skip the access when it is out of range, and
-// record the first failure (check code, index, bound) for att_kernel_debug_info.
-__device__ unsigned long long g_kernel_debug[3] = {0ull, 0ull, 0ull};
-#ifdef ATT_BOUNDS_CHECK
-__device__ __noinline__ void bounds_report(int code, long long a, long long b) {
-  atomicOr(&g_kernel_error, ATT_KERR_BOUNDS);
-  if (atomicCAS(&g_kernel_debug[0], 0ull, (unsigned long long)code) == 0ull) {
-    g_kernel_debug[1] = (unsigned long long)a;
-    g_kernel_debug[2] = (unsigned long long)b;
-  }
-}
-#define ATT_CHECK(cond, code, a, b) ((cond) ? true : (bounds_report((code), (a), (b)), false))
-#else
-#define ATT_CHECK(cond, code, a, b) true
-#endif
-
-// shared memory of one warp: per bead slot a 128-B brick, a neighbour-record
-// slot of rec_slot bytes, a 16-B moved-bead record and, in the modes that
-// accumulate dE/dmat, a 16-B ligand-frame record; the pair buffers of the
-// warp's teams (pairs_per_bead(K) u32 words per bead slot, plus S words of
-// padding per team so that teams start in different banks).
-// A team with more pairs than its buffer holds takes several windows; with
-// several beads per lane, 4 words per slot keep a block's shared memory small
-// enough for one more block per SM (13 % faster on 40-bead ligands at 2 beads
-// per lane, 51 % at 4) while most teams still need a single window.
-__host__ __device__ constexpr int pairs_per_bead(int K) { return K == 1 ? 8 : 4; }
-__host__ __device__ inline int rec_stride(int rec_slot) { return rec_slot ? rec_slot + 16 : 0; }
-__host__ __device__ inline size_t pair_buffer_bytes(int K) { return (size_t)32 * (pairs_per_bead(K) * K + 1) * 4; }
-// (the bead arms are held only by the modes that accumulate dE/dmat; the
-// others take the lever arm from the bead record)
-__host__ __device__ inline size_t warp_smem_bytes(int K, int rec_slot, bool arms = true) {
-  return (size_t)32 * K * (128 + rec_stride(rec_slot) + sizeof(BeadPos) + (arms ? sizeof(BeadArm) : 0)) +
-         pair_buffer_bytes(K);
 }
 
 template <int S>
@@ -260,7 +240,7 @@ __device__ __forceinline__ void pair_term_masked(const KParams& p, const KGrid& 
 template <int S, int K>
 __host__ __device__ constexpr int score_blocks_per_sm() { return K == 1 ? (S == 32 ? 6 : 5) : K == 2 ? 4 : 2; }
 
-template <int S, int K, int MODE>
+template <int S, int K, int MODE, bool ONE>
 __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kernel(const __grid_constant__ KParams p) {
   constexpr int P = 32 / S;      // poses per warp
   constexpr int NB = S * K;      // bead slots per pose
@@ -285,18 +265,28 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
   constexpr int ARM_BYTES = ACC9 ? 16 : 0;
   uint32_t* pbuf = reinterpret_cast<uint32_t*>(nrec + 32 * K * (RS + 16 + ARM_BYTES));
   const int tbase = slot * NB;  // this team's first bead record
-  const bool ref_grad = p.grad_mode == ATT_GRAD_REFERENCE;  // the pair loop and phase D compiled per mode
+  // the pair loop and phase D are compiled per gradient mode; the kernels over
+  // several grids hold the reference mode only (launch_score)
+  const bool ref_grad = !ONE || p.grad_mode == ATT_GRAD_REFERENCE;
   uint32_t* pb = pbuf + slot * (PB + S);  // this team's pair buffer
 
-  // Grid descriptors: copied from the parameters into shared memory with static
-  // parameter offsets only, so that the per-segment grid is picked by a
-  // dynamic index into shared memory (never into the parameter space).
-  __shared__ KGrid s_grid[ATT_MAX_GRIDS];
+  // Grid descriptors.  A launch over one grid (ONE: every call on a single
+  // receptor) reads its fields from the constant bank, as instruction operands.
+  // Several grids are copied into shared memory with static parameter offsets
+  // only, so that the per-segment grid is picked by a dynamic index into shared
+  // memory (never into the parameter space); there the fields cost ~29 of the
+  // 46 shared loads per pose and evaluation, on a data pipe 78 % busy, and the
+  // registers that hold them.  ONE against that, same results: 24-bead energrad
+  // of 65 536 poses 171 -> 131 us, 301-bead matrices 210 -> 185 us, forward and
+  // adjoint 614 -> 567 us, 40-bead minimiser 11.54 -> 10.72 ms, 18-30-bead
+  // minimiser 26.1 -> 24.9 ms, schema 10.16 -> 9.41 ms.
+  __shared__ KGrid s_grid[ONE ? 1 : ATT_MAX_GRIDS];
+  if constexpr (!ONE) {
 #pragma unroll
-  for (int g = 0; g < ATT_MAX_GRIDS; ++g)
-    if (threadIdx.x == g) s_grid[g] = p.grid[g];
-  __syncthreads();
-
+    for (int g = 0; g < ATT_MAX_GRIDS; ++g)
+      if (threadIdx.x == g) s_grid[g] = p.grid[g];
+    __syncthreads();
+  }
 
   // statistics (MODE_MIN): bead evaluations with a brick, list lookups, list
   // entries, brick copies, record copies
@@ -317,6 +307,16 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
     tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   }
 
+  auto next_tile = [&]() {
+    if (p.counter != nullptr) {
+      int t0 = 0;
+      if (lane == 0) t0 = atomicAdd(p.counter, 1);
+      tile = __shfl_sync(0xffffffffu, t0, 0);
+    } else {
+      tile += nwarps;
+    }
+  };
+
   while (tile < p.n_tiles) {
     const int si = find_segment(p, tile);
     AttSegment sg = p.segs[si];
@@ -327,12 +327,18 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
     const bool seg_ok = ((unsigned)sg.grid < (unsigned)p.n_grids) & ((unsigned)sg.lig < (unsigned)p.n_lig) &
                         (sg.pose0 >= 0) & (sg.n_poses >= 0) &
                         ((long long)sg.pose0 + sg.n_poses <= (long long)p.n_pose_rows);
+    // one launch of several over the same tiles: this one's grid only (the first
+    // one reports the bad segments)
+    if (ONE && (seg_ok ? sg.grid : 0) != p.grid_sel) {
+      next_tile();
+      continue;
+    }
     const int local = (tile - __ldg(p.seg_tile + si)) * P + slot;
     bool valid = seg_ok & (local >= 0) & (local < sg.n_poses);
     bool bad = !seg_ok;
     if (!seg_ok) sg.grid = sg.lig = sg.pose0 = sg.step0 = 0;
     const int b = sg.pose0 + (valid ? local : 0);
-    const KGrid& G = s_grid[sg.grid];
+    const KGrid& G = ONE ? p.grid[0] : s_grid[ONE ? 0 : sg.grid];
     int lig = sg.lig;
     if (p.pose_lig != nullptr && valid) {
       lig += __ldg(p.pose_lig + b);
@@ -1148,13 +1154,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
     if ((MODE == MODE_MIN || MODE == MODE_EVAL || QUAT) && valid && tl == 0 && p.status != nullptr)
       p.status[b] = status;
 
-    if (p.counter != nullptr) {
-      int t0 = 0;
-      if (lane == 0) t0 = atomicAdd(p.counter, 1);
-      tile = __shfl_sync(0xffffffffu, t0, 0);
-    } else {
-      tile += nwarps;
-    }
+    next_tile();
   }
 
   if (MODE == MODE_MIN && STATS_REGS && p.stats != nullptr) {
@@ -1169,61 +1169,38 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 }
 
 // ---------------------------------------------------------------------------
-// launch plumbing: (S, K) instantiations and their shared-memory needs
+// this part's (S, K) instantiations and error words
 // ---------------------------------------------------------------------------
-template <int MODE>
-struct KernelTable {
-  static const void* get(int S, int K) {
+template <int MODE, bool ONE>
+static const void* kernel_of_shape(int S, int K) {
 #define ATT_CASE(s_, k_) \
-  if (S == s_ && K == k_) return (const void*)score_kernel<s_, k_, MODE>;
-    ATT_CASE(32, 1) ATT_CASE(32, 2) ATT_CASE(32, 4) ATT_CASE(32, 8)
-    ATT_CASE(16, 1) ATT_CASE(16, 2) ATT_CASE(16, 4) ATT_CASE(16, 8)
-    ATT_CASE(8, 1) ATT_CASE(8, 2) ATT_CASE(8, 4) ATT_CASE(8, 8)
+  if (S == s_ && K == k_) return (const void*)score_kernel<s_, k_, MODE, ONE>;
+  ATT_CASE(32, 1) ATT_CASE(32, 2) ATT_CASE(32, 4) ATT_CASE(32, 8)
+  ATT_CASE(16, 1) ATT_CASE(16, 2) ATT_CASE(16, 4) ATT_CASE(16, 8)
+  ATT_CASE(8, 1) ATT_CASE(8, 2) ATT_CASE(8, 4) ATT_CASE(8, 8)
 #undef ATT_CASE
-    return nullptr;
-  }
-};
-
-static const void* kernel_of(int mode, int S, int K) {
-  switch (mode) {
-    case MODE_EVAL: return KernelTable<MODE_EVAL>::get(S, K);
-    case MODE_EVAL_MAT: return KernelTable<MODE_EVAL_MAT>::get(S, K);
-    case MODE_MIN: return KernelTable<MODE_MIN>::get(S, K);
-    case MODE_BWD: return KernelTable<MODE_BWD>::get(S, K);
-    case MODE_QUAT: return KernelTable<MODE_QUAT>::get(S, K);
-  }
   return nullptr;
 }
 
-int beads_per_lane(int S, int max_beads) {
-  const int need = (max_beads + S - 1) / S;
-  int K = 1;
-  while (K < need) K <<= 1;
-  return K <= ATT_MAX_BEADS_PER_LANE ? K : ATT_MAX_BEADS_PER_LANE;  // larger ligands run in chunks
+template <>
+const void* score_part_kernel<ATT_SCORE_PART>(int mode, int S, int K, bool one_grid) {
+#define ATT_MODE(m_) \
+  if (mode == m_) return one_grid ? kernel_of_shape<m_, true>(S, K) : kernel_of_shape<m_, false>(S, K);
+#if ATT_SCORE_PART == 0
+  ATT_MODE(MODE_EVAL) ATT_MODE(MODE_EVAL_MAT)
+#elif ATT_SCORE_PART == 1
+  ATT_MODE(MODE_MIN)
+#elif ATT_SCORE_PART == 2
+  ATT_MODE(MODE_BWD)
+#elif ATT_SCORE_PART == 3
+  ATT_MODE(MODE_QUAT)
+#endif
+#undef ATT_MODE
+  return nullptr;
 }
 
-size_t score_smem_bytes(int K, int threads, int rec_slot) {
-  return warp_smem_bytes(K, rec_slot) * (size_t)(threads / 32);
-}
-
-// the shared memory of one block of `mode` (without bead arms unless the mode
-// accumulates dE/dmat)
-static size_t mode_smem_bytes(int mode, int K, int threads, int rec_slot) {
-  const bool arms = mode == MODE_EVAL_MAT || mode == MODE_QUAT;
-  return warp_smem_bytes(K, rec_slot, arms) * (size_t)(threads / 32);
-}
-
-cudaError_t launch_score(const KParams& p, int mode, int S, int K, int blocks, int threads, cudaStream_t st) {
-  const void* k = kernel_of(mode, S, K);
-  if (k == nullptr) return cudaErrorInvalidValue;
-  const size_t smem = mode_smem_bytes(mode, K, threads, p.rec_slot);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  void* args[] = {const_cast<KParams*>(&p)};
-  return cudaLaunchKernel(k, dim3(blocks), dim3(threads), args, smem, st);
-}
-
-cudaError_t kernel_status(int* out, int clear, cudaStream_t st) {
+template <>
+cudaError_t score_part_status<ATT_SCORE_PART>(int* out, int clear, cudaStream_t st) {
   cudaError_t e = cudaMemcpyFromSymbolAsync(out, g_kernel_error, sizeof(int), 0, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaSuccess && clear && *out) {
@@ -1234,7 +1211,8 @@ cudaError_t kernel_status(int* out, int clear, cudaStream_t st) {
   return e;
 }
 
-cudaError_t kernel_debug_info(unsigned long long* out3, int clear, cudaStream_t st) {
+template <>
+cudaError_t score_part_debug<ATT_SCORE_PART>(unsigned long long* out3, int clear, cudaStream_t st) {
   cudaError_t e = cudaMemcpyFromSymbolAsync(out3, g_kernel_debug, 3 * sizeof(unsigned long long), 0,
                                             cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1244,15 +1222,6 @@ cudaError_t kernel_debug_info(unsigned long long* out3, int clear, cudaStream_t 
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   }
   return e;
-}
-
-cudaError_t occupancy_blocks(int mode, int S, int K, int threads, int rec_slot, int* blocks_per_sm) {
-  const void* k = kernel_of(mode, S, K);
-  if (k == nullptr) return cudaErrorInvalidValue;
-  const size_t smem = mode_smem_bytes(mode, K, threads, rec_slot);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, threads, smem);
 }
 
 }  // namespace att
