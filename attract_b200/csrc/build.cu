@@ -7,86 +7,210 @@
 namespace att {
 
 // ---------------------------------------------------------------------------
+// Receptor beads near a set of grid points
+// ---------------------------------------------------------------------------
+// The builders' sums and lists take a point's beads in index order, from those
+// within a radius.  A block first keeps the beads that come within the radius
+// of its points' bounding box -- in index order, so that sums and lists are
+// those of a loop over all beads -- and its threads look at these only.  The
+// box test takes the box's nearest coordinate on each axis through the same
+// rounded operations as the point test; those are monotone, so no bead that
+// passes at some point of the box fails it.
+
+// the rank of this thread among the block's threads that take, and their number
+// (w: THREADS / 32 words; a barrier has to lie between two uses)
+template <int THREADS>
+__device__ __forceinline__ int block_rank(bool take, unsigned* w, int& total) {
+  constexpr int W = THREADS / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned m = __ballot_sync(0xffffffffu, take);
+  if (lane == 0) w[warp] = __popc(m);
+  __syncthreads();
+  const unsigned c = lane < W ? w[lane] : 0u;
+  unsigned inc = c;
+#pragma unroll
+  for (int off = 1; off < W; off <<= 1) {
+    const unsigned t = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += t;
+  }
+  total = (int)__shfl_sync(0xffffffffu, inc, W - 1);
+  const unsigned before = __shfl_sync(0xffffffffu, inc - c, warp);
+  return (int)(before + __popc(m & ((1u << lane) - 1u)));
+}
+
+__device__ __forceinline__ float nearest_in(float r, float lo, float hi) { return fminf(fmaxf(r, lo), hi); }
+
+// ---------------------------------------------------------------------------
 // K3: energy + force voxels (test-calc-grid-energy.py:154-196, with forces)
 // ---------------------------------------------------------------------------
-constexpr int BUILD_THREADS = 256;
+// A block serves 4 x 8 x 8 grid points and 8 ligand types.  Bound by the FP64
+// pipe: per point, bead within the cutoff and type, 10 double operations (sums
+// are held in double), the distance, its reciprocal and the square root once for the 8
+// types.  The box keeps about 113 of 2500 beads (0.0093 / A^3, cutoff 10 A) of
+// which 39 reach a point; the pair rows are staged as doubles, read by a whole
+// warp at once.  2500 beads, 32 types, 1.44 M + 0.74 M points: 132.3 ms with
+// every bead tested per point and type, 2.1 ms with this kernel.
+constexpr int BP_THREADS = 256;
+constexpr int BP_TYPES = 8;    // ligand types per block
+constexpr int BP_STAGE = 32;   // beads whose pair rows are staged at a time
+constexpr int BP_LIST = 512;   // beads kept by the box before their sums are formed
 
-__global__ void __launch_bounds__(BUILD_THREADS)
+struct PairRowD {  // one (bead, ligand type) in double
+  double rc, ac, rc4, ac3;            // 4 rc, 3 ac
+  double ep, gp;                      // plateau energy, derivative
+  double cap, rmin2, ivor, shift;     // the general form: cap, sign, (ivor - 1) emin
+};
+
+__device__ __forceinline__ double dist2_d(double dx, double dy, double dz) { return fma(dz, dz, fma(dy, dy, dx * dx)); }
+
+__global__ void __launch_bounds__(BP_THREADS, 2)
 build_potential_kernel(AttGridGeom g, const float4* __restrict__ rec, int n_rec, const float4* __restrict__ pair,
-                       int n_rtypes, float cutoff2, int outer, float* __restrict__ out) {
-  __shared__ float4 srec[BUILD_THREADS];
-  const int lt = blockIdx.y;
+                       int n_rtypes, int n_ltypes, float cutoff2, int outer, int tiles_y, int tiles_z,
+                       float4* __restrict__ out) {
+  __shared__ float4 s_rec[BP_LIST];
+  __shared__ PairRowD s_row[BP_STAGE][BP_TYPES];
+  __shared__ double s_xyz[BP_STAGE][3];
+  __shared__ unsigned s_w[BP_THREADS / 32];
   const int nx = outer ? g.dim2[0] : g.dim[0];
   const int ny = outer ? g.dim2[1] : g.dim[1];
   const int nz = outer ? g.dim2[2] : g.dim[2];
-  const long long npts = (long long)nx * ny * nz;
-  const long long pt = (long long)blockIdx.x * BUILD_THREADS + threadIdx.x;
-  const bool live = pt < npts;
-  const int iz = (int)(pt % nz);
-  const int iy = (int)((pt / nz) % ny);
-  const int ix = (int)(pt / ((long long)nz * ny));
-  float px, py, pz;
-  if (!outer) {
-    px = g.origin[0] + ix * g.spacing;
-    py = g.origin[1] + iy * g.spacing;
-    pz = g.origin[2] + iz * g.spacing;
-  } else {
-    px = g.origin[0] + (2.f * ix - g.extension) * g.spacing;
-    py = g.origin[1] + (2.f * iy - g.extension) * g.spacing;
-    pz = g.origin[2] + (2.f * iz - g.extension) * g.spacing;
-  }
+  const int lt0 = blockIdx.y * BP_TYPES;
+  const int nt = min(BP_TYPES, n_ltypes - lt0);
+  const int tz = blockIdx.x % tiles_z, txy = blockIdx.x / tiles_z;
+  const int x0 = (txy / tiles_y) * 4, y0 = (txy % tiles_y) * 8, z0 = tz * 8;
+  // a warp serves 2 x 4 x 4 points: its points meet the same beads
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ix = x0 + ((warp >> 2) & 1) * 2 + (lane >> 4);
+  const int iy = y0 + ((warp >> 1) & 1) * 4 + ((lane >> 2) & 3);
+  const int iz = z0 + (warp & 1) * 4 + (lane & 3);
+  const bool live = ix < nx && iy < ny && iz < nz;
+  auto at = [&](int axis, int i) {
+    return !outer ? g.origin[axis] + i * g.spacing : g.origin[axis] + (2.f * i - g.extension) * g.spacing;
+  };
+  const double px = at(0, ix), py = at(1, iy), pz = at(2, iz);
+  const float lx = at(0, x0), hx = at(0, min(x0 + 3, nx - 1)), ly = at(1, y0), hy = at(1, min(y0 + 7, ny - 1));
+  const float lz = at(2, z0), hz = at(2, min(z0 + 7, nz - 1));
   const double p = g.plateau;
   const double p2 = p * p;
-  double e = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
-  const float4* prow = pair + (long long)lt * n_rtypes * 2;
-  for (int base = 0; base < n_rec; base += BUILD_THREADS) {
-    __syncthreads();
-    if (base + threadIdx.x < n_rec) srec[threadIdx.x] = rec[base + threadIdx.x];
-    __syncthreads();
-    const int m = min(BUILD_THREADS, n_rec - base);
-    if (!live) continue;
-    for (int k = 0; k < m; ++k) {
-      const float4 r = srec[k];
-      const double dx = (double)px - r.x, dy = (double)py - r.y, dz = (double)pz - r.z;
-      const double dsq = dx * dx + dy * dy + dz * dz;
-      if (!(dsq < cutoff2)) continue;
-      const int rt = __float_as_int(r.w);
-      if ((unsigned)rt >= (unsigned)n_rtypes) continue;
-      const float4 q0 = prow[rt * 2], q1 = prow[rt * 2 + 1];  // rc ac emin rmin2 | ivor eplat gplat rcap2
-      double scale;
-      if (dsq < p2) {
-        e += q1.y;
-        scale = dsq > 0.0 ? (double)q1.z * p / sqrt(dsq) : 0.0;
-      } else {
-        const double d2 = fmax(dsq, (double)q1.w);
-        const double rr2 = 1.0 / d2;
-        const double rr6 = rr2 * rr2 * rr2;
-        const double vlj = ((double)q0.x * rr2 - q0.y) * rr6;
-        const bool near = d2 < q0.w;
-        e += near ? vlj + ((double)q1.x - 1.0) * q0.z : (double)q1.x * vlj;
-        const double dv = rr6 * rr2 * (3.0 * q0.y - 4.0 * q0.x * rr2);
-        scale = (dsq < q1.w) ? 0.0 : (near ? dv : q1.x * dv);
-      }
-      fx -= 2.0 * scale * dx;
-      fy -= 2.0 * scale * dy;
-      fz -= 2.0 * scale * dz;
+  double e[BP_TYPES], fx[BP_TYPES], fy[BP_TYPES], fz[BP_TYPES];
+#pragma unroll
+  for (int t = 0; t < BP_TYPES; ++t) e[t] = fx[t] = fy[t] = fz[t] = 0.0;
+
+  int kept = 0;
+  for (int base = 0; base < n_rec; base += BP_THREADS) {
+    const int i = base + (int)threadIdx.x;
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool take = false;
+    if (i < n_rec) {
+      r = rec[i];
+      take = (unsigned)__float_as_int(r.w) < (unsigned)n_rtypes &&
+             dist2_d((double)nearest_in(r.x, lx, hx) - r.x, (double)nearest_in(r.y, ly, hy) - r.y,
+                     (double)nearest_in(r.z, lz, hz) - r.z) < cutoff2;
     }
+    int n = 0;
+    const int at_list = kept + block_rank<BP_THREADS>(take, s_w, n);
+    if (take) s_rec[at_list] = r;
+    kept += n;
+    __syncthreads();  // the list written, the warps' counts read
+    if (kept + BP_THREADS <= BP_LIST && base + BP_THREADS < n_rec) continue;
+    for (int k0 = 0; k0 < kept; k0 += BP_STAGE) {
+      const int m = min(BP_STAGE, kept - k0);
+      bool simple = true;
+      for (int q = threadIdx.x; q < m * BP_TYPES; q += BP_THREADS) {
+        const int k = q / BP_TYPES, t = q % BP_TYPES;
+        const float4 rk = s_rec[k0 + k];
+        if (t < 3) s_xyz[k][t] = t == 0 ? rk.x : t == 1 ? rk.y : rk.z;
+        if (t >= nt) continue;
+        const float4* prow = pair + ((long long)(lt0 + t) * n_rtypes + __float_as_int(rk.w)) * 2;
+        const float4 q0 = prow[0], q1 = prow[1];  // rc ac emin rmin2 | ivor eplat gplat rcap2
+        PairRowD& w = s_row[k][t];
+        w.rc = q0.x; w.ac = q0.y; w.rc4 = 4.0 * q0.x; w.ac3 = 3.0 * q0.y;
+        w.ep = q1.y; w.gp = q1.z;
+        w.cap = q1.w; w.rmin2 = q0.w; w.ivor = q1.x; w.shift = ((double)q1.x - 1.0) * q0.z;
+        simple &= q1.x == 1.f && w.shift == 0.0 && (double)q1.w <= p2;
+      }
+      // simple: attractive pairs (ivor = 1) with a cap inside the plateau only
+      const bool all_simple = __syncthreads_and(simple);
+      if (live) {
+        for (int k = 0; k < m; ++k) {
+          const double dx = px - s_xyz[k][0], dy = py - s_xyz[k][1], dz = pz - s_xyz[k][2];
+          const double dsq = dist2_d(dx, dy, dz);
+          if (!(dsq < cutoff2)) continue;
+          if (dsq < p2) {
+            const double pl = dsq > 0.0 ? -2.0 * p / sqrt(dsq) : 0.0;
+#pragma unroll
+            for (int t = 0; t < BP_TYPES; ++t) {
+              if (t < nt) {
+                const PairRowD& w = s_row[k][t];
+                const double sc = w.gp * pl;
+                e[t] += w.ep;
+                fx[t] = fma(sc, dx, fx[t]);
+                fy[t] = fma(sc, dy, fy[t]);
+                fz[t] = fma(sc, dz, fz[t]);
+              }
+            }
+          } else {
+            const double rr2 = 1.0 / dsq;
+            const double rr6 = rr2 * rr2 * rr2;
+            const double m8 = -2.0 * (rr6 * rr2);
+            if (all_simple) {
+#pragma unroll
+              for (int t = 0; t < BP_TYPES; ++t) {
+                if (t < nt) {
+                  const PairRowD& w = s_row[k][t];
+                  e[t] = fma(fma(w.rc, rr2, -w.ac), rr6, e[t]);
+                  const double sc = m8 * fma(-w.rc4, rr2, w.ac3);
+                  fx[t] = fma(sc, dx, fx[t]);
+                  fy[t] = fma(sc, dy, fy[t]);
+                  fz[t] = fma(sc, dz, fz[t]);
+                }
+              }
+            } else {
+#pragma unroll
+              for (int t = 0; t < BP_TYPES; ++t) {
+                if (t < nt) {
+                  const PairRowD& w = s_row[k][t];
+                  double r2 = rr2, r6 = rr6, d2 = dsq, sc = m8;
+                  if (dsq < w.cap) {  // constant below the cap: its energy, no force
+                    d2 = w.cap;
+                    r2 = 1.0 / d2;
+                    r6 = r2 * r2 * r2;
+                    sc = 0.0;
+                  }
+                  const double vlj = fma(w.rc, r2, -w.ac) * r6;
+                  const bool near = d2 < w.rmin2;
+                  e[t] += near ? vlj + w.shift : w.ivor * vlj;
+                  if (sc != 0.0) sc *= (near ? 1.0 : w.ivor) * fma(-w.rc4, r2, w.ac3);
+                  fx[t] = fma(sc, dx, fx[t]);
+                  fy[t] = fma(sc, dy, fy[t]);
+                  fz[t] = fma(sc, dz, fz[t]);
+                }
+              }
+            }
+          }
+        }
+      }
+      __syncthreads();  // the staged rows (and, after the last, the list) are read
+    }
+    kept = 0;
   }
   if (live) {
-    float4 v = make_float4((float)e, (float)fx, (float)fy, (float)fz);
-    reinterpret_cast<float4*>(out)[(long long)lt * npts + pt] = v;
+    const long long npts = (long long)nx * ny * nz, pt = ((long long)ix * ny + iy) * nz + iz;
+#pragma unroll
+    for (int t = 0; t < BP_TYPES; ++t)
+      if (t < nt) out[(lt0 + t) * npts + pt] = make_float4((float)e[t], (float)fx[t], (float)fy[t], (float)fz[t]);
   }
 }
 
 cudaError_t launch_build_potential(const AttGridGeom& g, const float* rec, int n_rec, const float* pair,
                                    int n_rtypes, int n_ltypes, float cutoff, int outer, float* out,
                                    cudaStream_t st) {
-  const long long npts = outer ? (long long)g.dim2[0] * g.dim2[1] * g.dim2[2]
-                               : (long long)g.dim[0] * g.dim[1] * g.dim[2];
-  dim3 grid((unsigned)((npts + BUILD_THREADS - 1) / BUILD_THREADS), (unsigned)n_ltypes);
-  build_potential_kernel<<<grid, BUILD_THREADS, 0, st>>>(g, reinterpret_cast<const float4*>(rec), n_rec,
-                                                         reinterpret_cast<const float4*>(pair), n_rtypes,
-                                                         cutoff * cutoff, outer, out);
+  const int* d = outer ? g.dim2 : g.dim;
+  const int tx = (d[0] + 3) / 4, ty = (d[1] + 7) / 8, tz = (d[2] + 7) / 8;
+  dim3 grid((unsigned)((long long)tx * ty * tz), (unsigned)((n_ltypes + BP_TYPES - 1) / BP_TYPES));
+  build_potential_kernel<<<grid, BP_THREADS, 0, st>>>(g, reinterpret_cast<const float4*>(rec), n_rec,
+                                                      reinterpret_cast<const float4*>(pair), n_rtypes, n_ltypes,
+                                                      cutoff * cutoff, outer, ty, tz, reinterpret_cast<float4*>(out));
   return cudaGetLastError();
 }
 
