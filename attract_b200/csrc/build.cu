@@ -472,26 +472,44 @@ cudaError_t launch_nb_fill(const AttGridGeom& g, const float* rec, int n_rec, fl
 }
 
 // CSR -> fixed-size records {inline entries, u16 count, u32 overflow index}:
-// the entries start the record, so that a reader takes four at a time in
-// 8-byte loads
-__global__ void nb_pack_kernel(const uint2* __restrict__ hdr, const uint16_t* __restrict__ list, long long nvox,
-                               int rec_bytes, unsigned char* __restrict__ out) {
-  const int inl = ATT_NB_INLINE(rec_bytes);
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nvox;
-       v += (long long)gridDim.x * blockDim.x) {
-    const uint2 h = hdr[v];
-    unsigned char* r = out + v * rec_bytes;
-    uint16_t* e = reinterpret_cast<uint16_t*>(r);
-    for (int i = 0; i < inl; ++i) e[i] = (i < (int)h.y) ? list[h.x + i] : (uint16_t)ATT_NB_EMPTY;
-    *reinterpret_cast<uint16_t*>(r + rec_bytes - 6) = (uint16_t)min(h.y, 65535u);
-    *reinterpret_cast<unsigned*>(r + rec_bytes - 4) = h.x + (unsigned)inl;
+// the entries start the record, so that a reader takes eight at a time in
+// 16-byte loads.  A thread forms a point's record in registers, 16 bytes at a
+// time.  Bound by the records' writes: 90.5 M points, 32-byte records: 7.50 ms
+// with 2-byte stores, 0.61 ms with these (2.9 GB written, 1.0 GB read).
+template <int RB>
+__global__ void __launch_bounds__(256)
+nb_pack_kernel(const uint2* __restrict__ hdr, const uint16_t* __restrict__ list, long long nvox,
+               uint4* __restrict__ out) {
+  constexpr int INL = ATT_NB_INLINE(RB);
+  const long long v = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (v >= nvox) return;
+  const uint2 h = hdr[v];
+  const uint16_t* l = list + h.x;
+  const unsigned cnt = h.y;
+  uint4* r = out + v * (RB / 16);
+  auto entry = [&](int i) -> unsigned {  // the i-th u16 of the record
+    return i == INL ? min(cnt, 65535u) : (unsigned)i < cnt ? ldg_u16(l + i) : (unsigned)ATT_NB_EMPTY;
+  };
+#pragma unroll
+  for (int q = 0; q < RB / 16; ++q) {
+    unsigned w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = q * 8 + k * 2;
+      w[k] = i > INL ? h.x + (unsigned)INL : entry(i) | entry(i + 1) << 16;
+    }
+    r[q] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
 cudaError_t launch_nb_pack(const uint32_t* hdr, const uint16_t* list, long long nvox, int rec_bytes, void* out,
                            cudaStream_t st) {
-  nb_pack_kernel<<<148 * 8, 256, 0, st>>>(reinterpret_cast<const uint2*>(hdr), list, nvox, rec_bytes,
-                                          reinterpret_cast<unsigned char*>(out));
+  const uint2* h = reinterpret_cast<const uint2*>(hdr);
+  uint4* o = reinterpret_cast<uint4*>(out);
+  const unsigned blocks = (unsigned)((nvox + 255) / 256);
+  if (rec_bytes == 32) nb_pack_kernel<32><<<blocks, 256, 0, st>>>(h, list, nvox, o);
+  else if (rec_bytes == 64) nb_pack_kernel<64><<<blocks, 256, 0, st>>>(h, list, nvox, o);
+  else nb_pack_kernel<128><<<blocks, 256, 0, st>>>(h, list, nvox, o);
   return cudaGetLastError();
 }
 
