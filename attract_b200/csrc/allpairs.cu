@@ -3,30 +3,40 @@
 // test-energy.py:46-58 (delta over all pairs, nonbon of every d^2, summed per
 // structure), with ATTRACT's --rcut as an optional distance cutoff.
 //
-// One block of 8 warps per pose (grid-stride over poses).  The receptor streams
-// through shared memory in tiles of AP_TILE beads; a warp takes one ligand bead
-// at a time against 32 consecutive receptor beads per step (conflict-free
-// 16-byte shared loads).  The pair-parameter row depends on the receptor type:
-// a lane keeps the last row it loaded and reloads only when the type changes,
-// so a receptor sorted by type (the host wrapper sorts it) reads each row once
-// per run of equal types instead of once per pair.  Per bead, the warp's lane
-// sums (energy and force, float) are reduced with shuffles and added to the
-// bead's accumulator in shared memory (double); the torque -- or x (x) g for the
-// 4x4 form -- is formed once per bead from its total force, and the block sums
-// the beads in double.
+// An item is one ligand bead of one pose.  A lane serves two items at a time in
+// packed float operations (or four, in two packed sets), and a warp's lanes meet
+// the same receptor bead together: it is one broadcast from shared memory, the
+// type test is uniform, and the pair rows of a lane's items stay in registers
+// while the receptor type lasts (the host wrapper sorts the receptor by type).
+// A lane sums an item's energy and force over at most 64 receptor beads in
+// float, then in double.  The receptor is split over `rw` groups of the block's
+// warps and over the `cl` blocks of a cluster; a pose's sums over its beads,
+// groups and blocks (the latter over distributed shared memory, in rank order)
+// are formed in double.  plan() weighs the splits: a library of poses fills the
+// GPU with whole receptors, a handful of poses needs every split there is.
+//
+// Bound by the FMA pipe (a packed operation takes it twice as long as a plain
+// one: 19 of them per two pairs) and by issue: 17.5 instructions per pair at four items per
+// lane, the pipe 63 % and the issue slots 56 % busy, against 52.7 for a warp that met 32
+// receptor beads at once (a row test and shuffles of its own per bead).  2500 x
+// 24 beads: 16 384 poses 1958 -> 890 us (1.1 T pairs/s), 10 poses 48 us on one block each -> below
+// the 18 us that the call takes on the host.
+#include <cooperative_groups.h>
 #include <math.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
 namespace att {
 int report_error(int code, const char* msg);
+namespace cg = cooperative_groups;
 
 constexpr int AP_THREADS = 256;
 constexpr int AP_WARPS = AP_THREADS / 32;
-constexpr int AP_TILE = 2048;   // receptor beads per shared-memory tile (32 KB)
-constexpr int AP_BEADS = 512;   // ligand beads per pass (their accumulators: 16 KB)
-constexpr size_t AP_SMEM = (size_t)AP_TILE * sizeof(float4) + (size_t)AP_BEADS * 4 * sizeof(double) +
-                           (size_t)AP_WARPS * 13 * sizeof(double);
+constexpr int AP_TILE = 1024;    // receptor beads in shared memory (32 B each), over the block's groups
+constexpr int AP_FLUSH = 64;     // receptor beads summed in float
+constexpr int AP_POSES = 128;    // poses of a block
 
 struct AllPairsParams {
   const float4* rec;   // [n_rec] x, y, z, receptor type (int bits)
@@ -37,190 +47,424 @@ struct AllPairsParams {
   float* grad;         // [B][6] or [B][16], may be NULL
   float rcut2;         // <= 0: no cutoff
   int n_rec, n_lig, n_poses, pose_format, n_rtypes, n_ltypes;
+  int rw, cl;          // receptor groups per block, blocks per cluster
+  int pb, nb;          // poses per block, ligand beads per pass (all of them unless pb = 1)
 };
 
-// block-wide double sum of v[0..n); result valid in thread 0
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) red[warp * NV + k] = v[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < AP_WARPS; ++w) s += red[w * NV + k];
-      v[k] = s;
-    }
-  }
-  __syncthreads();
+// two floats in one register pair: every operation rounds as the plain one
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-
-// 1/d2: the approximate reciprocal refined by one Newton step (within 1 ulp)
-__device__ __forceinline__ float recip_nr(float d2) {
+__device__ __forceinline__ void upk(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d2));
-  return r * fmaf(-d2, r, 2.f);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
+// a pose's row-vector rotation M (X = x M + t) and, for Euler poses, what its
+// gradient takes of the angles
+struct PoseM {
+  float m[9], t[3], sphi, cphi, spsi, cpsi;
+};
+__device__ __forceinline__ PoseM load_pose(const AllPairsParams& p, int b) {
+  PoseM q;
+  q.sphi = q.spsi = 0.f;
+  q.cphi = q.cpsi = 1.f;
+  if (p.pose_format == 1) {
+    const float* P = p.pose + (long long)b * 16;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) q.m[r * 3 + c] = __ldg(P + r * 4 + c);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) q.t[c] = __ldg(P + 12 + c);
+  } else {
+    const float* P = p.pose + (long long)b * 6;
+    float sth, cth;
+    sincosf(__ldg(P + 0), &q.sphi, &q.cphi);
+    sincosf(__ldg(P + 1), &q.spsi, &q.cpsi);
+    sincosf(__ldg(P + 2), &sth, &cth);
+    // column-form Q = Rz(phi) Ry(psi) Rz(-theta); the row-vector M is its transpose
+    q.m[0] = q.cphi * q.cpsi * cth + q.sphi * sth;
+    q.m[1] = q.sphi * q.cpsi * cth - q.cphi * sth;
+    q.m[2] = -q.spsi * cth;
+    q.m[3] = q.cphi * q.cpsi * sth - q.sphi * cth;
+    q.m[4] = q.sphi * q.cpsi * sth + q.cphi * cth;
+    q.m[5] = -q.spsi * sth;
+    q.m[6] = q.cphi * q.spsi;
+    q.m[7] = q.sphi * q.spsi;
+    q.m[8] = q.cpsi;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) q.t[c] = __ldg(P + 3 + c);
+  }
+  return q;
+}
+
+constexpr int ap_slots(int NP) { return AP_WARPS * 64 * NP; }  // items of a block, over its receptor groups
+constexpr size_t ap_smem(int NP) {
+  return (size_t)(AP_TILE + 1) * 2 * sizeof(float4) + (size_t)ap_slots(NP) * 4 * sizeof(double) +
+         (size_t)AP_POSES * (13 * sizeof(double) + sizeof(PoseM));
+}
+
+// NP: packed pairs of items per lane; CUT: rcut; GRAD: the gradient too
+template <int NP, bool CUT, bool GRAD>
 __global__ void __launch_bounds__(AP_THREADS) allpairs_kernel(const __grid_constant__ AllPairsParams p) {
-  extern __shared__ __align__(16) unsigned char ap_smem[];
-  float4* s_rec = reinterpret_cast<float4*>(ap_smem);
-  double* s_acc = reinterpret_cast<double*>(ap_smem + (size_t)AP_TILE * sizeof(float4));  // [AP_BEADS][4]
-  double* red = s_acc + AP_BEADS * 4;
+  extern __shared__ __align__(16) unsigned char ap_smem_raw[];
+  float4* s_rec = reinterpret_cast<float4*>(ap_smem_raw);                // [AP_TILE + 1][2]: -x -x -y -y, -z -z type -
+  double* s_item = reinterpret_cast<double*>(s_rec + (AP_TILE + 1) * 2);  // [group][E, Gx, Gy, Gz][item]
+  double* s_sum = s_item + ap_slots(NP) * 4;                              // [pose][13]
+  PoseM* s_m = reinterpret_cast<PoseM*>(s_sum + AP_POSES * 13);           // [pose]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool mat = p.pose_format == 1;
-  for (int b = blockIdx.x; b < p.n_poses; b += gridDim.x) {
-    // pose -> row-vector rotation M (X = x M + t) and, for Euler poses, the angles
-    float m[9], t[3], sphi = 0.f, cphi = 1.f, spsi = 0.f, cpsi = 1.f;
-    if (mat) {
-      const float* P = p.pose + (long long)b * 16;
+  const int rank = (int)(blockIdx.x % (unsigned)p.cl);
+  const int pose0 = (int)(blockIdx.x / (unsigned)p.cl) * p.pb;
+  const int np = min(p.pb, p.n_poses - pose0);
+  const int iw = AP_WARPS / p.rw, slots = iw * 64 * NP;
+  const int group = warp / iw, first = (warp % iw) * 64 * NP + lane;  // this lane's items: first + 32 k
+  const int lo = (int)((long long)p.n_rec * rank / p.cl), hi = (int)((long long)p.n_rec * (rank + 1) / p.cl);
+  auto bound = [&](int g) { return lo + (int)((long long)(hi - lo) * g / p.rw); };
+  const int tile = AP_TILE / p.rw, longest = (hi - lo + p.rw - 1) / p.rw;
+  const int g0 = bound(group), g1 = bound(group + 1);
+
+  for (int k = threadIdx.x; k < np; k += AP_THREADS) s_m[k] = load_pose(p, pose0 + k);
+  for (int k = threadIdx.x; k < np * 13; k += AP_THREADS) s_sum[k] = 0.0;
+
+  for (int i0 = 0; i0 < p.n_lig; i0 += p.nb) {
+    const int nb = min(p.nb, p.n_lig - i0);
+    const int items = np * nb;
+    __syncthreads();  // the poses are there; the last pass's sums are read
+    // this lane's items: moved beads, ligand types (-1: no item, or no pair row)
+    f2 X[NP], Y[NP], Z[NP];
+    int lt[2 * NP];
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+    for (int k = 0; k < NP; ++k) {
+      float c[2][3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) m[r * 3 + c] = __ldg(P + r * 4 + c);
+      for (int h = 0; h < 2; ++h) {
+        const int it = first + 32 * (2 * k + h);
+        c[h][0] = c[h][1] = c[h][2] = 0.f;
+        lt[2 * k + h] = -1;
+        if (it < items) {
+          const float4 x = __ldg(p.lig + i0 + it % nb);
+          const PoseM& q = s_m[it / nb];
+          const int t = __float_as_int(x.w);
+          lt[2 * k + h] = (unsigned)t < (unsigned)p.n_ltypes ? t : -1;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) t[c] = __ldg(P + 12 + c);
-    } else {
-      const float* P = p.pose + (long long)b * 6;
-      float sth, cth;
-      sincosf(__ldg(P + 0), &sphi, &cphi);
-      sincosf(__ldg(P + 1), &spsi, &cpsi);
-      sincosf(__ldg(P + 2), &sth, &cth);
-      // column-form Q = Rz(phi) Ry(psi) Rz(-theta); the row-vector M is its transpose
-      const float q00 = cphi * cpsi * cth + sphi * sth, q01 = cphi * cpsi * sth - sphi * cth, q02 = cphi * spsi;
-      const float q10 = sphi * cpsi * cth - cphi * sth, q11 = sphi * cpsi * sth + cphi * cth, q12 = sphi * spsi;
-      const float q20 = -spsi * cth, q21 = -spsi * sth, q22 = cpsi;
-      m[0] = q00; m[1] = q10; m[2] = q20;
-      m[3] = q01; m[4] = q11; m[5] = q21;
-      m[6] = q02; m[7] = q12; m[8] = q22;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) t[c] = __ldg(P + 3 + c);
+          for (int d = 0; d < 3; ++d) c[h][d] = fmaf(x.x, q.m[d], fmaf(x.y, q.m[3 + d], fmaf(x.z, q.m[6 + d], q.t[d])));
+        }
+      }
+      X[k] = pk(c[0][0], c[1][0]);
+      Y[k] = pk(c[0][1], c[1][1]);
+      Z[k] = pk(c[0][2], c[1][2]);
     }
-    // energy, force and the lever-arm sums (torque, or x (x) g for the 4x4 form)
-    double acc[13];
+    // its items' sums in double: E, Gx, Gy, Gz, each a row of the group's items
+    double* sums = s_item + (size_t)group * slots * 4 + first;
 #pragma unroll
-    for (int k = 0; k < 13; ++k) acc[k] = 0.0;
-    for (int i0 = 0; i0 < p.n_lig; i0 += AP_BEADS) {
-      const int nb = min(AP_BEADS, p.n_lig - i0);
-      for (int k = threadIdx.x; k < nb * 4; k += AP_THREADS) s_acc[k] = 0.0;
-      for (int j0 = 0; j0 < p.n_rec; j0 += AP_TILE) {
-        const int nt = min(AP_TILE, p.n_rec - j0);
-        __syncthreads();  // the previous tile has been read
-        for (int j = threadIdx.x; j < nt; j += AP_THREADS) s_rec[j] = __ldg(p.rec + j0 + j);
-        __syncthreads();
-        for (int i = i0 + warp; i < i0 + nb; i += AP_WARPS) {  // warp-uniform
-          const float4 x = __ldg(p.lig + i);
-          const int lt = __float_as_int(x.w);
-          if ((unsigned)lt >= (unsigned)p.n_ltypes) continue;  // no pair table row: contributes nothing
-          const float X = fmaf(x.x, m[0], fmaf(x.y, m[3], fmaf(x.z, m[6], t[0])));
-          const float Y = fmaf(x.x, m[1], fmaf(x.y, m[4], fmaf(x.z, m[7], t[1])));
-          const float Z = fmaf(x.x, m[2], fmaf(x.y, m[5], fmaf(x.z, m[8], t[2])));
-          const float4* prow = p.pair + (size_t)lt * p.n_rtypes * 2;
-          float e = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-          int cur = -1;
-          float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;  // rc, ac, emin, rmin2 / ivor, eplat, -, rcap2
-          for (int j = lane; j < nt; j += 32) {
-            const float4 r = s_rec[j];
-            const int rt = __float_as_int(r.w);
-            const float dx = X - r.x, dy = Y - r.y, dz = Z - r.z;
-            const float dsq = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            const bool hit = ((unsigned)rt < (unsigned)p.n_rtypes) & ((p.rcut2 <= 0.f) | (dsq < p.rcut2));
-            const int rtc = hit ? rt : 0;
-            if (rtc != cur) {  // a new receptor type: its row
-              ldg_f4x2(prow + rtc * 2, p0, p1);
-              cur = rtc;
+    for (int k = 0; k < 2 * NP; ++k)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sums[c * slots + 32 * k] = 0.0;
+    const bool idle = __all_sync(0xffffffffu, first >= items);
+    // the pair rows of the lane's items with the current receptor type
+    f2 rc[NP], ac[NP], rc8[NP], ac6[NP];
+    float cap[2 * NP];
+    bool simple = true, use = false;
+    int cur = -1;
+#pragma unroll
+    for (int k = 0; k < 2 * NP; ++k) cap[k] = 0.f;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) rc[k] = ac[k] = rc8[k] = ac6[k] = 0ull;
+
+    for (int t0 = 0; t0 < longest; t0 += tile) {
+      __syncthreads();  // the previous tile has been read
+      for (int k = threadIdx.x; k < AP_TILE; k += AP_THREADS) {
+        const int g = k / tile, j = bound(g) + t0 + k % tile;
+        if (g < p.rw && j < bound(g + 1)) {
+          const float4 r = __ldg(p.rec + j);
+          s_rec[2 * k] = make_float4(-r.x, -r.x, -r.y, -r.y);
+          s_rec[2 * k + 1] = make_float4(-r.z, -r.z, r.w, 0.f);
+        }
+      }
+      __syncthreads();
+      const int len = idle ? 0 : min(tile, g1 - g0 - t0);
+      const float4* rec = s_rec + 2 * group * tile;
+      for (int c0 = 0; c0 < len; c0 += AP_FLUSH) {
+        const int c1 = min(len, c0 + AP_FLUSH);
+        f2 e[NP], gx[NP], gy[NP], gz[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) e[k] = gx[k] = gy[k] = gz[k] = 0ull;
+        for (int j = c0; j < c1;) {
+          float4 A = rec[2 * j], B = rec[2 * j + 1];
+          const int rt = __float_as_int(B.z);
+          if (rt != cur) {  // a new receptor type: the rows of this lane's items
+            cur = rt;
+            use = (unsigned)rt < (unsigned)p.n_rtypes;  // (no row: the bead contributes nothing)
+            simple = true;
+            if (use) {
+              float v[2 * NP][2];
+#pragma unroll
+              for (int k = 0; k < 2 * NP; ++k) {
+                const float4* row = p.pair + ((size_t)max(lt[k], 0) * p.n_rtypes + rt) * 2;
+                const float4 q0 = __ldg(row), q1 = __ldg(row + 1);
+                v[k][0] = q0.x;
+                v[k][1] = q0.y;
+                cap[k] = q1.w;
+                // attractive, no shift: the plain form on both sides of the minimum
+                simple &= q1.x == 1.f && q1.y == 0.f && isfinite(q0.z);
+              }
+#pragma unroll
+              for (int k = 0; k < NP; ++k) {
+                rc[k] = pk(v[2 * k][0], v[2 * k + 1][0]);
+                ac[k] = pk(v[2 * k][1], v[2 * k + 1][1]);
+                rc8[k] = pk(8.f * v[2 * k][0], 8.f * v[2 * k + 1][0]);
+                ac6[k] = pk(6.f * v[2 * k][1], 6.f * v[2 * k + 1][1]);
+              }
+              simple = __all_sync(0xffffffffu, simple);
             }
-            const float d2 = fmaxf(dsq, p1.w);
-            const float rr2 = recip_nr(d2);
-            const float rr6 = rr2 * rr2 * rr2;
-            const float vlj = fmaf(p0.x, rr2, -p0.y) * rr6;
-            const bool near = d2 < p0.w;
-            const float en = near ? fmaf(p1.x - 1.f, p0.z, vlj) : p1.x * vlj;
-            float gm2 = rr6 * rr2 * fmaf(-8.f * p0.x, rr2, 6.f * p0.y);  // 2 dnonbon/d(d^2)
-            gm2 = near ? gm2 : p1.x * gm2;
-            gm2 = (dsq < p1.w) ? 0.f : gm2;
-            const float gf = hit ? gm2 : 0.f;
-            e += hit ? en - p1.y : 0.f;
-            gx = fmaf(gf, dx, gx);
-            gy = fmaf(gf, dy, gy);
-            gz = fmaf(gf, dz, gz);
           }
+          // the receptor beads of one type
+          auto run = [&](auto simple_form) {
+            constexpr bool SIMPLE = decltype(simple_form)::value;
+            const f2 two = pk(2.f, 2.f);
+            float emin[2 * NP], rmin2[2 * NP], ivor[2 * NP], epl[2 * NP];  // what only the general form takes
+            if (!SIMPLE) {
 #pragma unroll
-          for (int off = 16; off >= 1; off >>= 1) {
-            e += __shfl_xor_sync(0xffffffffu, e, off);
-            gx += __shfl_xor_sync(0xffffffffu, gx, off);
-            gy += __shfl_xor_sync(0xffffffffu, gy, off);
-            gz += __shfl_xor_sync(0xffffffffu, gz, off);
-          }
-          if (lane == 0) {  // bead i belongs to this warp alone
-            double* a = s_acc + (i - i0) * 4;
-            a[0] += e;
-            a[1] += gx;
-            a[2] += gy;
-            a[3] += gz;
+              for (int k = 0; k < 2 * NP; ++k) {
+                const float4* row = p.pair + ((size_t)max(lt[k], 0) * p.n_rtypes + cur) * 2;
+                const float4 q0 = __ldg(row), q1 = __ldg(row + 1);
+                emin[k] = q0.z;
+                rmin2[k] = q0.w;
+                ivor[k] = q1.x;
+                epl[k] = q1.y;
+              }
+            }
+            do {
+              const float4 A1 = rec[2 * j + 2], B1 = rec[2 * j + 3];  // (the tile has one more)
+              const f2 nx = pk(A.x, A.y), ny = pk(A.z, A.w), nz = pk(B.x, B.y);
+#pragma unroll
+              for (int k = 0; k < NP; ++k) {
+                const f2 dx = add2(X[k], nx), dy = add2(Y[k], ny), dz = add2(Z[k], nz);
+                const f2 dsq = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                float q0, q1;
+                upk(dsq, q0, q1);
+                const float d0 = fmaxf(q0, cap[2 * k]), d1 = fmaxf(q1, cap[2 * k + 1]);
+                const f2 d2 = pk(d0, d1);
+                // n = -1/d2: the approximate reciprocal and one Newton step (within 1 ulp)
+                const f2 a = pk(rcp_approx(-d0), rcp_approx(-d1));
+                const f2 n = mul2(a, fma2(d2, a, two));
+                const f2 n3 = mul2(mul2(n, n), n);
+                const f2 u = fma2(rc[k], n, ac[k]);                         // (rc r^-2 - ac) r^-6 = u n3
+                f2 gm = mul2(mul2(n3, n), fma2(rc8[k], n, ac6[k]));  // 2 dnonbon/d(d^2)
+                float g0_, g1_;
+                upk(gm, g0_, g1_);
+                if (SIMPLE && !CUT) {
+                  e[k] = fma2(u, n3, e[k]);
+                } else {
+                  float e0, e1;
+                  upk(mul2(u, n3), e0, e1);
+                  if (!SIMPLE) {
+                    const bool b0 = d0 < rmin2[2 * k], b1 = d1 < rmin2[2 * k + 1];
+                    e0 = (b0 ? fmaf(ivor[2 * k] - 1.f, emin[2 * k], e0) : ivor[2 * k] * e0) - epl[2 * k];
+                    e1 = (b1 ? fmaf(ivor[2 * k + 1] - 1.f, emin[2 * k + 1], e1) : ivor[2 * k + 1] * e1) - epl[2 * k + 1];
+                    g0_ = b0 ? g0_ : ivor[2 * k] * g0_;
+                    g1_ = b1 ? g1_ : ivor[2 * k + 1] * g1_;
+                  }
+                  if (CUT) {
+                    e0 = q0 < p.rcut2 ? e0 : 0.f;
+                    e1 = q1 < p.rcut2 ? e1 : 0.f;
+                  }
+                  e[k] = add2(e[k], pk(e0, e1));
+                }
+                if (GRAD) {
+                  g0_ = (CUT ? (q0 < cap[2 * k]) | !(q0 < p.rcut2) : q0 < cap[2 * k]) ? 0.f : g0_;
+                  g1_ = (CUT ? (q1 < cap[2 * k + 1]) | !(q1 < p.rcut2) : q1 < cap[2 * k + 1]) ? 0.f : g1_;
+                  gm = pk(g0_, g1_);
+                  gx[k] = fma2(gm, dx, gx[k]);
+                  gy[k] = fma2(gm, dy, gy[k]);
+                  gz[k] = fma2(gm, dz, gz[k]);
+                }
+              }
+              A = A1;
+              B = B1;
+              ++j;
+            } while (j < c1 && __float_as_int(B.z) == cur);
+          };
+          if (!use) ++j;
+          else if (simple) run(std::true_type{});
+          else run(std::false_type{});
+        }
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+          const f2 v[4] = {e[k], gx[k], gy[k], gz[k]};
+#pragma unroll
+          for (int c = 0; c < (GRAD ? 4 : 1); ++c) {
+            float a, b;
+            upk(v[c], a, b);
+            sums[c * slots + 64 * k] += a;
+            sums[c * slots + 64 * k + 32] += b;
           }
         }
       }
-      __syncthreads();  // every warp's accumulators written (or just cleared)
-      // per bead of this pass: energy, force and its lever-arm terms
-      for (int i = i0 + threadIdx.x; i < i0 + nb; i += AP_THREADS) {
-        const double* a = s_acc + (i - i0) * 4;
-        const double e = a[0], gx = a[1], gy = a[2], gz = a[3];
-        const float4 x = __ldg(p.lig + i);
-        acc[0] += e;
-        acc[1] += gx;
-        acc[2] += gy;
-        acc[3] += gz;
-        if (mat) {  // dE/dM[r][c] = sum_i x_r g_c
-          const double xr[3] = {x.x, x.y, x.z}, gc[3] = {gx, gy, gz};
-#pragma unroll
-          for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) acc[4 + r * 3 + c] += xr[r] * gc[c];
-        } else {  // torque about the pose centre: (X - t) x g, X - t = x M
-          const double ax = fmaf(x.x, m[0], fmaf(x.y, m[3], x.z * m[6]));
-          const double ay = fmaf(x.x, m[1], fmaf(x.y, m[4], x.z * m[7]));
-          const double az = fmaf(x.x, m[2], fmaf(x.y, m[5], x.z * m[8]));
-          acc[4] += ay * gz - az * gy;
-          acc[5] += az * gx - ax * gz;
-          acc[6] += ax * gy - ay * gx;
-        }
-      }
-      __syncthreads();  // the accumulators are read before the next pass clears them
     }
-    block_sum<13>(acc, red);
-    if (threadIdx.x == 0) {
-      p.energy[b] = (float)acc[0];
-      if (p.grad != nullptr) {
-        if (mat) {
-          float* g = p.grad + (long long)b * 16;
 #pragma unroll
-          for (int r = 0; r < 3; ++r) {
+    for (int k = 0; k < 2 * NP; ++k)
+      if (lt[k] < 0) {  // no pair row: the bead contributes nothing
 #pragma unroll
-            for (int c = 0; c < 3; ++c) g[r * 4 + c] = (float)acc[4 + r * 3 + c];
-            g[r * 4 + 3] = 0.f;
+        for (int c = 0; c < 4; ++c) sums[c * slots + 32 * k] = 0.0;
+      }
+    __syncthreads();
+    // a pose's sums over its beads and the receptor groups: 8 lanes per pose
+    for (int q0 = 0; q0 < np; q0 += AP_THREADS / 8) {
+      const int q = q0 + (int)threadIdx.x / 8;
+      double acc[13];
+#pragma unroll
+      for (int k = 0; k < 13; ++k) acc[k] = 0.0;
+      if (q < np) {
+        const PoseM& pm = s_m[q];
+        for (int i = threadIdx.x & 7; i < nb; i += 8) {
+          double v[4] = {0.0, 0.0, 0.0, 0.0};
+          for (int g = 0; g < p.rw; ++g) {
+            const double* a = s_item + (size_t)g * slots * 4 + q * nb + i;
+#pragma unroll
+            for (int k = 0; k < (GRAD ? 4 : 1); ++k) v[k] += a[k * slots];
           }
-          g[12] = (float)acc[1]; g[13] = (float)acc[2]; g[14] = (float)acc[3]; g[15] = 0.f;
-        } else {
-          // dE/d(angle_k) = w_k . torque with w_phi = (0,0,1), w_psi = (-sin phi, cos phi, 0),
-          // w_theta = -(cos phi sin psi, sin phi sin psi, cos psi)
-          float* g = p.grad + (long long)b * 6;
-          const double tx = acc[4], ty = acc[5], tz = acc[6];
-          g[0] = (float)tz;
-          g[1] = (float)(-sphi * tx + cphi * ty);
-          g[2] = (float)(-(cphi * spsi * tx + sphi * spsi * ty + cpsi * tz));
-          g[3] = (float)acc[1]; g[4] = (float)acc[2]; g[5] = (float)acc[3];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[k] += v[k];
+          if (GRAD) {
+            const float4 x = __ldg(p.lig + i0 + i);
+            if (mat) {  // dE/dM[r][c] = sum_i x_r g_c
+              const double xr[3] = {x.x, x.y, x.z};
+#pragma unroll
+              for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[4 + r * 3 + c] += xr[r] * v[1 + c];
+            } else {  // torque about the pose centre: (X - t) x g, X - t = x M
+              double a[3];
+#pragma unroll
+              for (int d = 0; d < 3; ++d) a[d] = fmaf(x.x, pm.m[d], fmaf(x.y, pm.m[3 + d], x.z * pm.m[6 + d]));
+              acc[4] += a[1] * v[3] - a[2] * v[2];
+              acc[5] += a[2] * v[1] - a[0] * v[3];
+              acc[6] += a[0] * v[2] - a[1] * v[1];
+            }
+          }
         }
+      }
+      const int nv = !GRAD ? 1 : mat ? 13 : 7;
+#pragma unroll
+      for (int k = 0; k < 13; ++k)
+        if (k < nv) {
+#pragma unroll
+          for (int off = 4; off >= 1; off >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+          if (q < np && (threadIdx.x & 7) == 0) s_sum[q * 13 + k] += acc[k];
+        }
+    }
+  }
+  __syncthreads();
+  if (p.cl > 1) {  // the other blocks' sums, in rank order
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    if (rank == 0)
+      for (int k = threadIdx.x; k < np * 13; k += AP_THREADS) {
+        double v = s_sum[k];
+        for (int r = 1; r < p.cl; ++r) v += *cluster.map_shared_rank(s_sum + k, r);
+        s_sum[k] = v;
+      }
+    cluster.sync();
+    if (rank != 0) return;
+  }
+  for (int q = threadIdx.x; q < np; q += AP_THREADS) {
+    const double* a = s_sum + q * 13;
+    const long long b = pose0 + q;
+    p.energy[b] = (float)a[0];
+    if (GRAD) {
+      if (mat) {
+        float* g = p.grad + b * 16;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) g[r * 4 + c] = (float)a[4 + r * 3 + c];
+          g[r * 4 + 3] = 0.f;
+        }
+        g[12] = (float)a[1]; g[13] = (float)a[2]; g[14] = (float)a[3]; g[15] = 0.f;
+      } else {
+        // dE/d(angle_k) = w_k . torque with w_phi = (0,0,1), w_psi = (-sin phi, cos phi, 0),
+        // w_theta = -(cos phi sin psi, sin phi sin psi, cos psi)
+        const PoseM& m = s_m[q];
+        float* g = p.grad + b * 6;
+        const double tx = a[4], ty = a[5], tz = a[6];
+        g[0] = (float)tz;
+        g[1] = (float)(-m.sphi * tx + m.cphi * ty);
+        g[2] = (float)(-(m.cphi * m.spsi * tx + m.sphi * m.spsi * ty + m.cpsi * tz));
+        g[3] = (float)a[1]; g[4] = (float)a[2]; g[5] = (float)a[3];
       }
     }
   }
+}
+
+typedef void (*ApKernel)(AllPairsParams);
+template <int NP>
+static ApKernel ap_kernel(bool cut, bool grad) {
+  return cut ? (grad ? allpairs_kernel<NP, true, true> : allpairs_kernel<NP, true, false>)
+             : (grad ? allpairs_kernel<NP, false, true> : allpairs_kernel<NP, false, false>);
+}
+
+// The split of a call: packed pairs per lane, receptor groups per block, blocks
+// per cluster.  The time is taken as waves of resident blocks (3 per SM at one
+// packed pair per lane, 2 at two, by registers).  A block costs its steps (a receptor bead
+// against a lane's items; 1.9 at two packed pairs), 80 steps for its start and sums, 20
+// per pass over the ligand and 4 per block of its cluster; 2 and 3 blocks on an
+// SM advance at 1.6 and 2.0 times the rate of one (1.7 for 2 at two packed
+// pairs).  Fitted to all 32 splits of 16 calls of 150-5000 receptor beads, 3-300
+// ligand beads and 30-65 536 poses: the split taken is within 3 % of the fastest on average
+// (at most 10 %), where the slowest is 3 to 10 times slower.
+struct ApPlan {
+  int np, rw, cl, pb, nb;
+};
+static ApPlan ap_plan(long long n_poses, int n_lig, int n_rec, int sms) {
+  ApPlan best = {1, 1, 1, 1, 1};
+  double best_t = 1e300;
+  for (int np = 1; np <= 2; ++np)
+    for (int rw = 1; rw <= AP_WARPS; rw *= 2)
+      for (int cl = 1; cl <= 8; cl *= 2) {
+        const int slots = (AP_WARPS / rw) * 64 * np;
+        ApPlan q = {np, rw, cl, 1, slots};
+        if (n_lig <= slots) {
+          q.pb = slots / n_lig < AP_POSES ? slots / n_lig : AP_POSES;
+          q.nb = n_lig;
+        }
+        if (q.pb > n_poses) q.pb = (int)n_poses;
+        const double passes = (double)(((long long)n_lig + q.nb - 1) / q.nb);
+        const double cost = passes * ((np == 1 ? 1.0 : 1.9) * n_rec / (rw * cl) + 20.0) + 80.0 + 4.0 * cl;
+        const double rate[4] = {1.0, 1.0, np == 1 ? 1.6 : 1.7, 2.0};
+        const int resident = np == 1 ? 3 : 2;
+        const long long blocks = (n_poses + q.pb - 1) / q.pb * cl;
+        const long long full = blocks / ((long long)resident * sms), rest = blocks - full * resident * sms;
+        const int last = (int)((rest + sms - 1) / sms);  // blocks on an SM in the last wave
+        const double t = cost * ((double)full * resident / rate[resident] + last / rate[last]);
+        if (t < best_t) {
+          best_t = t;
+          best = q;
+        }
+      }
+  return best;
 }
 
 }  // namespace att
@@ -259,14 +503,28 @@ extern "C" int att_allpairs_energy(const float* rec_dev, int n_rec, const float*
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaError_t e = cudaFuncSetAttribute(allpairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AP_SMEM);
+  const ApPlan plan = ap_plan(n_poses, n_lig, n_rec, sms);
+  p.rw = plan.rw;
+  p.cl = plan.cl;
+  p.pb = plan.pb;
+  p.nb = plan.nb;
+  const bool cut = p.rcut2 > 0.f, grad = grad_dev != nullptr;
+  const ApKernel kernel = plan.np == 1 ? ap_kernel<1>(cut, grad) : ap_kernel<2>(cut, grad);
+  const size_t smem = plan.np == 1 ? ap_smem(1) : ap_smem(2);
+  cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return report_error(ATT_E_CUDA, cudaGetErrorString(e));
-  int per_sm = 1;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, allpairs_kernel, AP_THREADS, AP_SMEM);
-  if (e != cudaSuccess) return report_error(ATT_E_CUDA, cudaGetErrorString(e));
-  const int blocks = (int)min((long long)n_poses, (long long)sms * max(per_sm, 1));
-  allpairs_kernel<<<blocks, AP_THREADS, AP_SMEM, (cudaStream_t)stream>>>(p);
-  e = cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)plan.cl;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(((long long)n_poses + plan.pb - 1) / plan.pb * plan.cl));
+  cfg.blockDim = dim3(AP_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = (cudaStream_t)stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = plan.cl > 1 ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) return report_error(ATT_E_CUDA, cudaGetErrorString(e));
   return ATT_OK;
 }
