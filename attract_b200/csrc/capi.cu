@@ -11,6 +11,7 @@ cudaError_t occupancy_blocks(int mode, int S, int K, int threads, int rec_slot, 
 cudaError_t kernel_status(int* out, int clear, cudaStream_t st);
 cudaError_t kernel_debug_info(unsigned long long* out3, int clear, cudaStream_t st);
 int beads_per_lane(int S, int max_beads);
+int mode_beads_per_lane(int mode, int S, int max_beads);
 size_t score_smem_bytes(int K, int threads, int rec_slot);
 cudaError_t launch_build_potential(const AttGridGeom& g, const float* rec, int n_rec, const float* pair,
                                    int n_rtypes, int n_ltypes, float cutoff, int outer, float* out,
@@ -167,7 +168,7 @@ static int make_kgrid(const AttGrid* a, int gi, KGrid* k) {
   return ATT_OK;
 }
 
-static int fill_common(KParams* p, const AttGrid* grids, int n_grids, const AttLigands* ligs,
+static int fill_common(KParams* p, int mode, const AttGrid* grids, int n_grids, const AttLigands* ligs,
                        const AttSegment* segs, int n_segs, const int* seg_tile, int n_tiles, int n_pose_rows,
                        const float* pose,
                        const int* pose_lig, const AttEvalCfg* cfg, const AttLaunchCfg* launch, int* S, int* K,
@@ -190,7 +191,8 @@ static int fill_common(KParams* p, const AttGrid* grids, int n_grids, const AttL
   REQUIRE(ligs->max_beads >= 1, "ligands: max_beads = %d", ligs->max_beads);
   REQUIRE(ligs->n_beads >= ligs->max_beads, "ligands: n_beads = %d < max_beads = %d", ligs->n_beads,
           ligs->max_beads);
-  *K = beads_per_lane(s, ligs->max_beads);
+  const int all = beads_per_lane(s, ligs->max_beads);  // beads per lane that hold a whole ligand
+  *K = mode_beads_per_lane(mode, s, ligs->max_beads);
   int t = (launch && launch->block_threads) ? launch->block_threads : 128;
   REQUIRE(t == 32 || t == 64 || t == 96 || t == 128, "block_threads = %d (32, 64, 96 or 128)", t);
   *threads = t;
@@ -204,12 +206,16 @@ static int fill_common(KParams* p, const AttGrid* grids, int n_grids, const AttL
   p->rec_slot = rec_slot;
   REQUIRE(!launch || launch->test_flags == 0, "AttLaunchCfg.test_flags is reserved and must be 0");
   p->test_flags = 0;
-  if (!(launch && launch->block_threads)) {  // default: the largest block whose shared memory fits
+  if (launch && launch->block_threads) {  // a caller's block has to hold whole ligands
+    REQUIRE(score_smem_bytes(all, t, rec_slot) <= kDynSmemLimit,
+            "%d threads x %d beads per lane need %zu B of shared memory", t, all, score_smem_bytes(all, t, rec_slot));
+  } else {  // default: the largest block whose shared memory fits
     while (t > 32 && score_smem_bytes(*K, t, rec_slot) > kDynSmemLimit) t -= 32;
     *threads = t;
   }
-  REQUIRE(score_smem_bytes(*K, t, rec_slot) <= kDynSmemLimit,
-          "%d threads x %d beads per lane need %zu B of shared memory", t, *K, score_smem_bytes(*K, t, rec_slot));
+  REQUIRE(score_smem_bytes(*K, *threads, rec_slot) <= kDynSmemLimit,
+          "%d threads x %d beads per lane need %zu B of shared memory", *threads, *K,
+          score_smem_bytes(*K, *threads, rec_slot));
   p->lig_beads = reinterpret_cast<const float4*>(ligs->beads);
   p->lig_off = ligs->offset;
   p->segs = segs;
@@ -235,7 +241,7 @@ extern "C" int att_energrad(const AttGrid* grids, int n_grids, const AttLigands*
                             int* status_dev, const AttLaunchCfg* launch, void* stream) {
   KParams p;
   int S = 8, K = 1, threads = 128;
-  int rc = fill_common(&p, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_dev, pose_lig_dev,
+  int rc = fill_common(&p, MODE_EVAL, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_dev, pose_lig_dev,
                        cfg, launch, &S, &K, &threads);
   if (rc) return rc;
   REQUIRE(energy_dev != nullptr || n_tiles == 0, "energy output is NULL");
@@ -282,7 +288,7 @@ extern "C" int att_minimise(const AttGrid* grids, int n_grids, const AttLigands*
   REQUIRE(cfg != nullptr, "adam cfg is NULL");
   KParams p;
   int S = 8, K = 1, threads = 128;
-  int rc = fill_common(&p, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_in_dev,
+  int rc = fill_common(&p, MODE_MIN, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_in_dev,
                        pose_lig_dev, &cfg->eval, launch, &S, &K, &threads);
   if (rc) return rc;
   REQUIRE(cfg->eval.pose_format == 0, "att_minimise takes Euler poses (pose_format 0)");
@@ -309,7 +315,7 @@ extern "C" int att_minimise(const AttGrid* grids, int n_grids, const AttLigands*
   if (n_tiles == 0) return ATT_OK;
   int blocks = 0;
   rc = persistent_blocks(MODE_MIN, S, K, threads, p.rec_slot,
-                         n_grids == 1 || p.grad_mode == ATT_GRAD_ANALYTIC, launch, n_tiles, &blocks);
+                         n_grids == 1 || (K > 1 && p.grad_mode == ATT_GRAD_ANALYTIC), launch, n_tiles, &blocks);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = launch_score(p, MODE_MIN, S, K, blocks, threads, st);
@@ -325,7 +331,7 @@ extern "C" int att_minimise_schema(const AttGrid* grids, int n_grids, const AttL
   REQUIRE(cfg != nullptr, "schema cfg is NULL");
   KParams p;
   int S = 8, K = 1, threads = 128;
-  int rc = fill_common(&p, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_in_dev,
+  int rc = fill_common(&p, MODE_QUAT, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_in_dev,
                        pose_lig_dev, &cfg->eval, launch, &S, &K, &threads);
   if (rc) return rc;
   REQUIRE(cfg->n_stages >= 1 && cfg->n_stages <= ATT_MAX_STAGES, "n_stages = %d (1..%d)", cfg->n_stages,
@@ -359,7 +365,7 @@ extern "C" int att_minimise_schema(const AttGrid* grids, int n_grids, const AttL
   if (n_tiles == 0) return ATT_OK;
   int blocks = 0;
   rc = persistent_blocks(MODE_QUAT, S, K, threads, p.rec_slot,
-                         n_grids == 1 || p.grad_mode == ATT_GRAD_ANALYTIC, launch, n_tiles, &blocks);
+                         n_grids == 1 || (K > 1 && p.grad_mode == ATT_GRAD_ANALYTIC), launch, n_tiles, &blocks);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = launch_score(p, MODE_QUAT, S, K, blocks, threads, st);
@@ -374,7 +380,7 @@ extern "C" int att_energrad_backward(const AttGrid* grids, int n_grids, const At
                                      float* dgrid_outer_dev, const AttLaunchCfg* launch, void* stream) {
   KParams p;
   int S = 8, K = 1, threads = 128;
-  int rc = fill_common(&p, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_dev, pose_lig_dev,
+  int rc = fill_common(&p, MODE_BWD, grids, n_grids, ligs, segs_dev, n_segs, seg_tile_dev, n_tiles, n_pose_rows, pose_dev, pose_lig_dev,
                        cfg, launch, &S, &K, &threads);
   if (rc) return rc;
   REQUIRE(cfg->pose_format == 0, "att_energrad_backward takes Euler poses (pose_format 0)");

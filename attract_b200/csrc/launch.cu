@@ -22,6 +22,20 @@ int beads_per_lane(int S, int max_beads) {
   return K <= ATT_MAX_BEADS_PER_LANE ? K : ATT_MAX_BEADS_PER_LANE;  // larger ligands run in chunks
 }
 
+// A minimiser keeps every bead's brick and record in shared memory from step to
+// step, so its lanes hold all of a ligand's beads.  A single evaluation copies each
+// once whatever its chunk: one bead per lane leaves room for 24 warps per SM (16, 8 and 4 at
+// 2, 4 and 8 beads per lane) to cover the copies' latency.  32 lanes: 40 beads,
+// 20 000 poses 78 -> 69 us; 100 beads, 8000 poses 97 -> 65; 200 beads, 5000 poses
+// 191 -> 76; 301 beads, 3000 matrices 184 -> 64; the adjoint of 100 beads, 8000 poses
+// 129 -> 105.  With at most 8 warps of work per SM the chunks' latencies add up instead:
+// 301 beads, 300 poses 20 -> 30 us, 100 beads 9.2 -> 13.3, less than the 13.5 us that a
+// call takes on the host.  One rule for all sizes keeps a pose's energy the same to the bit
+// in any batch.
+int mode_beads_per_lane(int mode, int S, int max_beads) {
+  return mode == MODE_MIN || mode == MODE_QUAT ? beads_per_lane(S, max_beads) : 1;
+}
+
 size_t score_smem_bytes(int K, int threads, int rec_slot) {
   return warp_smem_bytes(K, rec_slot) * (size_t)(threads / 32);
 }
@@ -33,27 +47,33 @@ static size_t mode_smem_bytes(int mode, int K, int threads, int rec_slot) {
   return warp_smem_bytes(K, rec_slot, arms) * (size_t)(threads / 32);
 }
 
+// lets a kernel use `bytes` of dynamic shared memory; 48 KB need no leave (a
+// driver call less for small launches)
+static cudaError_t allow_smem(const void* k, size_t bytes) {
+  return bytes <= 48 * 1024 ? cudaSuccess
+                            : cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 static cudaError_t launch_one(const KParams& p, int mode, int S, int K, bool one_grid, int blocks, int threads,
                               cudaStream_t st) {
   const void* k = kernel_of(mode, S, K, one_grid);
   if (k == nullptr) return cudaErrorInvalidValue;
   const size_t smem = mode_smem_bytes(mode, K, threads, p.rec_slot);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, smem);
   if (e == cudaSuccess && p.counter != nullptr) e = cudaMemsetAsync(p.counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<KParams*>(&p)};
   return cudaLaunchKernel(k, dim3(blocks), dim3(threads), args, smem, st);
 }
 
-// One grid, or the reference gradient on several: one launch.  The analytic
-// gradient on several grids: one launch per grid over the same tiles, each
-// skipping the other grids' segments.  (The kernels over several grids hold the
-// reference mode only: the 32-lane, two-beads-per-lane evaluation compiled with
-// both modes reported a misaligned address in the analytic one, on lists that
-// continue in the CSR tail, where the bounds-checked build of the same source
-// found every index and alignment right.)
+// One launch, but for the analytic gradient of a minimiser over several grids with
+// several beads per lane: one per grid over the same tiles, each skipping the other grids'
+// segments.  (Those kernels hold the reference mode only.  Compiled with both, a
+// 32-lane, two-beads-per-lane evaluation over two grids reported a misaligned address in
+// the analytic mode, where the bounds-checked build of the same source found
+// every index and alignment right.)
 cudaError_t launch_score(const KParams& p, int mode, int S, int K, int blocks, int threads, cudaStream_t st) {
-  if (p.n_grids == 1 || p.grad_mode == ATT_GRAD_REFERENCE)
+  if (p.n_grids == 1 || K == 1 || p.grad_mode == ATT_GRAD_REFERENCE)
     return launch_one(p, mode, S, K, p.n_grids == 1, blocks, threads, st);
   KParams q = p;
   for (int g = 0; g < p.n_grids; ++g) {
@@ -94,7 +114,7 @@ cudaError_t occupancy_blocks(int mode, int S, int K, int threads, int rec_slot, 
   const void* k = kernel_of(mode, S, K, one_grid);
   if (k == nullptr) return cudaErrorInvalidValue;
   const size_t smem = mode_smem_bytes(mode, K, threads, rec_slot);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, threads, smem);
 }

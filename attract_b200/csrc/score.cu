@@ -265,9 +265,9 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
   constexpr int ARM_BYTES = ACC9 ? 16 : 0;
   uint32_t* pbuf = reinterpret_cast<uint32_t*>(nrec + 32 * K * (RS + 16 + ARM_BYTES));
   const int tbase = slot * NB;  // this team's first bead record
-  // the pair loop and phase D are compiled per gradient mode; the kernels over
-  // several grids hold the reference mode only (launch_score)
-  const bool ref_grad = !ONE || p.grad_mode == ATT_GRAD_REFERENCE;
+  // the pair loop and phase D are compiled per gradient mode; with several beads
+  // per lane the kernels over several grids hold the reference mode only (launch_score)
+  const bool ref_grad = (!ONE && K > 1) || p.grad_mode == ATT_GRAD_REFERENCE;
   uint32_t* pb = pbuf + slot * (PB + S);  // this team's pair buffer
 
   // Grid descriptors.  A launch over one grid (ONE: every call on a single
@@ -1175,9 +1175,12 @@ template <int MODE, bool ONE>
 static const void* kernel_of_shape(int S, int K) {
 #define ATT_CASE(s_, k_) \
   if (S == s_ && K == k_) return (const void*)score_kernel<s_, k_, MODE, ONE>;
-  ATT_CASE(32, 1) ATT_CASE(32, 2) ATT_CASE(32, 4) ATT_CASE(32, 8)
-  ATT_CASE(16, 1) ATT_CASE(16, 2) ATT_CASE(16, 4) ATT_CASE(16, 8)
-  ATT_CASE(8, 1) ATT_CASE(8, 2) ATT_CASE(8, 4) ATT_CASE(8, 8)
+  ATT_CASE(32, 1) ATT_CASE(16, 1) ATT_CASE(8, 1)
+  if constexpr (MODE == MODE_MIN || MODE == MODE_QUAT) {  // (mode_beads_per_lane)
+    ATT_CASE(32, 2) ATT_CASE(32, 4) ATT_CASE(32, 8)
+    ATT_CASE(16, 2) ATT_CASE(16, 4) ATT_CASE(16, 8)
+    ATT_CASE(8, 2) ATT_CASE(8, 4) ATT_CASE(8, 8)
+  }
 #undef ATT_CASE
   return nullptr;
 }
