@@ -46,8 +46,8 @@ class AllPairs:
         if p2.device != self.device or p2.dtype != torch.float32 or not p2.is_contiguous():
             raise ValueError("poses must be a contiguous float32 tensor on the receptor's device")
         B = len(p2)
-        E = torch.empty(B, dtype=torch.float32, device=self.device)
-        G = torch.empty((B, 16 if mat else 6), dtype=torch.float32, device=self.device) if grad else None
+        E = p2.new_empty(B)
+        G = p2.new_empty((B, 16 if mat else 6)) if grad else None
         rc = _lib.load().att_allpairs_energy(_lib.ptr(self.rec) if self.n_rec else None, self.n_rec,
                                              _lib.ptr(self.lig), self.n_lig, _lib.ptr(p2), B, 1 if mat else 0,
                                              _lib.ptr(self.pair), self.ff.n_rtypes, self.ff.n_ltypes,

@@ -29,12 +29,8 @@ class EvalOptions:
     def to_c(self, pose_format: int = 0) -> _lib.AttEvalCfg:
         if self.grad_mode not in ("reference", "analytic"):
             raise ValueError(f"grad_mode {self.grad_mode!r}")
-        c = _lib.AttEvalCfg()
-        c.grad_mode = _lib.ATT_GRAD_REFERENCE if self.grad_mode == "reference" else _lib.ATT_GRAD_ANALYTIC
-        c.flags = _lib.ATT_FLAG_TRILINEAR_QUIRK if self.quirk else 0
-        c.gravity = float(self.gravity)
-        c.pose_format = pose_format
-        return c
+        return _lib.AttEvalCfg(_lib.ATT_GRAD_REFERENCE if self.grad_mode == "reference" else _lib.ATT_GRAD_ANALYTIC,
+                               _lib.ATT_FLAG_TRILINEAR_QUIRK if self.quirk else 0, float(self.gravity), pose_format)
 
 
 @dataclass
@@ -63,10 +59,7 @@ class LaunchShape:
     test_flags: int = 0       # reserved: 0
 
     def to_c(self) -> _lib.AttLaunchCfg:
-        c = _lib.AttLaunchCfg()
-        c.lanes_per_pose, c.block_threads, c.blocks = self.lanes_per_pose, self.block_threads, self.blocks
-        c.test_flags = self.test_flags
-        return c
+        return _lib.AttLaunchCfg(self.lanes_per_pose, self.block_threads, self.blocks, self.test_flags)
 
     @property
     def poses_per_warp(self) -> int:
@@ -81,8 +74,14 @@ class Segment(NamedTuple):
     pose0: int | None = None  # first pose in the pose array (None: packed in segment order)
 
 
+# the current stream's handle without a Stream object around it (3 us of a small call's 19)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream):
     if stream is None:
+        if _raw_stream is not None:
+            return _raw_stream(torch._C._cuda_getDevice())
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, torch.cuda.Stream):
         return stream.cuda_stream
@@ -190,9 +189,9 @@ def energrad(wl: Workload, poses: torch.Tensor, opts: EvalOptions | None = None,
     wl.check_poses(p2, 16 if mat else 6)
     B = wl.n_poses
     if out is None:
-        E = torch.empty(B, dtype=torch.float32, device=wl.device)
-        G = torch.empty((B, 16 if mat else 6), dtype=torch.float32, device=wl.device) if grad else None
-        S = torch.empty(B, dtype=torch.int32, device=wl.device)
+        E = p2.new_empty(B)
+        G = p2.new_empty((B, 16 if mat else 6)) if grad else None
+        S = p2.new_empty(B, dtype=torch.int32)
     else:
         E, G, S = out
     if pose_lig is not None:
@@ -303,7 +302,7 @@ class MinimiseScratch:
     def __init__(self, n_poses: int, device):
         self.energy = torch.empty(max(n_poses, 1), dtype=torch.float32, device=device)[:n_poses]
         self.status = torch.empty(max(n_poses, 1), dtype=torch.int32, device=device)[:n_poses]
-        self.counter = torch.zeros(1, dtype=torch.int32, device=device)
+        self.counter = torch.empty(1, dtype=torch.int32, device=device)  # (every launch clears it)
 
 
 def energrad_backward(wl: Workload, poses: torch.Tensor, dL_dE: torch.Tensor, opts: EvalOptions | None = None,
