@@ -17,25 +17,32 @@ namespace att {
 // rounded operations as the point test; those are monotone, so no bead that
 // passes at some point of the box fails it.
 
-// the rank of this thread among the block's threads that take, and their number
-// (w: THREADS / 32 words; a barrier has to lie between two uses)
+// The ranks of this thread's elements among those that the block's threads take,
+// and their number.  Element k of a thread is the (THREADS k + thread)-th: ranks
+// follow the index.  (w: 32 words; a barrier has to lie between two uses)
 template <int THREADS>
-__device__ __forceinline__ int block_rank(bool take, unsigned* w, int& total) {
-  constexpr int W = THREADS / 32;
+__device__ __forceinline__ void block_ranks(const bool (&take)[1024 / THREADS], unsigned* w, int (&rank)[1024 / THREADS],
+                                            int& total) {
+  constexpr int W = THREADS / 32, N = 1024 / THREADS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned m = __ballot_sync(0xffffffffu, take);
-  if (lane == 0) w[warp] = __popc(m);
+  unsigned m[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    m[k] = __ballot_sync(0xffffffffu, take[k]);
+    if (lane == 0) w[k * W + warp] = __popc(m[k]);
+  }
   __syncthreads();
-  const unsigned c = lane < W ? w[lane] : 0u;
+  const unsigned c = w[lane];
   unsigned inc = c;
 #pragma unroll
-  for (int off = 1; off < W; off <<= 1) {
+  for (int off = 1; off < 32; off <<= 1) {
     const unsigned t = __shfl_up_sync(0xffffffffu, inc, off);
     if (lane >= off) inc += t;
   }
-  total = (int)__shfl_sync(0xffffffffu, inc, W - 1);
-  const unsigned before = __shfl_sync(0xffffffffu, inc - c, warp);
-  return (int)(before + __popc(m & ((1u << lane) - 1u)));
+  total = (int)__shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    rank[k] = (int)(__shfl_sync(0xffffffffu, inc - c, k * W + warp) + __popc(m[k] & ((1u << lane) - 1u)));
 }
 
 __device__ __forceinline__ float nearest_in(float r, float lo, float hi) { return fminf(fmaxf(r, lo), hi); }
@@ -49,11 +56,12 @@ __device__ __forceinline__ float nearest_in(float r, float lo, float hi) { retur
 // types.  The box keeps about 113 of 2500 beads (0.0093 / A^3, cutoff 10 A) of
 // which 39 reach a point; the pair rows are staged as doubles, read by a whole
 // warp at once.  2500 beads, 32 types, 1.44 M + 0.74 M points: 132.3 ms with
-// every bead tested per point and type, 2.1 ms with this kernel.
+// every bead tested per point and type, 1.96 ms with this kernel.
 constexpr int BP_THREADS = 256;
 constexpr int BP_TYPES = 8;    // ligand types per block
 constexpr int BP_STAGE = 32;   // beads whose pair rows are staged at a time
-constexpr int BP_LIST = 512;   // beads kept by the box before their sums are formed
+constexpr int BP_LIST = 1408;  // beads kept by the box before their sums are formed
+constexpr int BP_STEP = 1024;  // beads tested against the box between two barriers
 
 struct PairRowD {  // one (bead, ligand type) in double
   double rc, ac, rc4, ac3;            // 4 rc, 3 ac
@@ -70,7 +78,7 @@ build_potential_kernel(AttGridGeom g, const float4* __restrict__ rec, int n_rec,
   __shared__ float4 s_rec[BP_LIST];
   __shared__ PairRowD s_row[BP_STAGE][BP_TYPES];
   __shared__ double s_xyz[BP_STAGE][3];
-  __shared__ unsigned s_w[BP_THREADS / 32];
+  __shared__ unsigned s_w[32];
   const int nx = outer ? g.dim2[0] : g.dim[0];
   const int ny = outer ? g.dim2[1] : g.dim[1];
   const int nz = outer ? g.dim2[2] : g.dim[2];
@@ -97,22 +105,29 @@ build_potential_kernel(AttGridGeom g, const float4* __restrict__ rec, int n_rec,
   for (int t = 0; t < BP_TYPES; ++t) e[t] = fx[t] = fy[t] = fz[t] = 0.0;
 
   int kept = 0;
-  for (int base = 0; base < n_rec; base += BP_THREADS) {
-    const int i = base + (int)threadIdx.x;
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    bool take = false;
-    if (i < n_rec) {
-      r = rec[i];
-      take = (unsigned)__float_as_int(r.w) < (unsigned)n_rtypes &&
-             dist2_d((double)nearest_in(r.x, lx, hx) - r.x, (double)nearest_in(r.y, ly, hy) - r.y,
-                     (double)nearest_in(r.z, lz, hz) - r.z) < cutoff2;
+  for (int base = 0; base < n_rec; base += BP_STEP) {
+    constexpr int N = BP_STEP / BP_THREADS;
+    float4 r[N];
+    bool take[N];
+    int rank[N], n = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int i = base + k * BP_THREADS + (int)threadIdx.x;
+      take[k] = i < n_rec;
+      if (take[k]) r[k] = rec[i];
     }
-    int n = 0;
-    const int at_list = kept + block_rank<BP_THREADS>(take, s_w, n);
-    if (take) s_rec[at_list] = r;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      take[k] = take[k] && (unsigned)__float_as_int(r[k].w) < (unsigned)n_rtypes &&
+                dist2_d((double)nearest_in(r[k].x, lx, hx) - r[k].x, (double)nearest_in(r[k].y, ly, hy) - r[k].y,
+                        (double)nearest_in(r[k].z, lz, hz) - r[k].z) < cutoff2;
+    block_ranks<BP_THREADS>(take, s_w, rank, n);
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (take[k]) s_rec[kept + rank[k]] = r[k];
     kept += n;
     __syncthreads();  // the list written, the warps' counts read
-    if (kept + BP_THREADS <= BP_LIST && base + BP_THREADS < n_rec) continue;
+    if (kept + BP_STEP <= BP_LIST && base + BP_STEP < n_rec) continue;
     for (int k0 = 0; k0 < kept; k0 += BP_STAGE) {
       const int m = min(BP_STAGE, kept - k0);
       bool simple = true;
@@ -262,65 +277,111 @@ __device__ __forceinline__ bool box_reached(const PointBox& q, const float4& r, 
 
 // A block serves NB_POINTS consecutive points, NB_THREADS at a time.
 constexpr int NB_THREADS = 512, NB_POINTS = 4096, NB_SUB = NB_POINTS / NB_THREADS;
-constexpr int NB_LIST = 1024;  // beads kept by the block's box before its points look at them
+constexpr int NB_LIST = 1536;  // beads kept by the block's box before its points look at them
+constexpr int NB_STEP = 1024;  // beads tested against the box between two barriers
 
 // Calls hit(s, bead, n) for every bead within the radius of this thread's s-th
 // point v0 + NB_THREADS * s + thread, in index order; n is what the previous call for
 // the point returned (0 at first), and s_n[s][thread] the last one.  The block
 // keeps the beads near its points (about 75 of 2500 on the x4 list grid, whose
 // blocks are nine rows 100 A long), a warp those near its 32 points (about 11),
-// and only these are tested per point.
+// and only these are tested per point.  A warp within one row of z (nearly all)
+// has one x and y: fl(fl(dx dx) + fl(dy dy)) is formed once per bead and warp.
 template <class Hit>
 __device__ __forceinline__ void near_beads(const AttGridGeom& g, const float4* __restrict__ rec, int n_rec, float r2,
                                            long long nvox, unsigned (&s_n)[NB_SUB][NB_THREADS], Hit hit) {
   __shared__ float4 s_rec[NB_LIST];
   __shared__ unsigned short s_idx[NB_LIST];
-  __shared__ unsigned s_w[NB_THREADS / 32];
+  __shared__ unsigned s_w[32];
   const long long v0 = (long long)blockIdx.x * NB_POINTS, last = nvox - 1;
   const int lane = threadIdx.x & 31;
   const PointBox block = box_of(g, index_of(g, v0), index_of(g, min(v0 + NB_POINTS - 1, last)));
 #pragma unroll
   for (int s = 0; s < NB_SUB; ++s) s_n[s][threadIdx.x] = 0u;
   int kept = 0;
-  for (int base = 0; base < n_rec; base += NB_THREADS) {
-    const int i = base + (int)threadIdx.x;
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    bool take = false;
-    if (i < n_rec) {
-      r = rec[i];
-      take = box_reached(block, r, r2);
+  for (int base = 0; base < n_rec; base += NB_STEP) {
+    constexpr int N = NB_STEP / NB_THREADS;
+    float4 r[N];
+    bool take[N];
+    int rank[N], n = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int i = base + k * NB_THREADS + (int)threadIdx.x;
+      take[k] = i < n_rec;
+      if (take[k]) r[k] = rec[i];
     }
-    int n = 0;
-    const int k = kept + block_rank<NB_THREADS>(take, s_w, n);
-    if (take) {
-      s_rec[k] = r;
-      s_idx[k] = (unsigned short)i;
-    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) take[k] = take[k] && box_reached(block, r[k], r2);
+    block_ranks<NB_THREADS>(take, s_w, rank, n);
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (take[k]) {
+        s_rec[kept + rank[k]] = r[k];
+        s_idx[kept + rank[k]] = (unsigned short)(base + k * NB_THREADS + (int)threadIdx.x);
+      }
     kept += n;
     __syncthreads();  // the list written, the warps' counts read
-    if (kept == 0 || (kept + NB_THREADS <= NB_LIST && base + NB_THREADS < n_rec)) continue;
+    if (kept == 0 || (kept + NB_STEP <= NB_LIST && base + NB_STEP < n_rec)) continue;
+    int3 me = index_of(g, min(v0 + threadIdx.x, last));
     for (int s = 0; s < NB_SUB; ++s) {
       const long long w0 = v0 + s * NB_THREADS + (threadIdx.x & ~31);
       if (w0 > last) break;
-      const int3 me = index_of(g, min(w0 + lane, last));
-      const float x = coord_of(g, 0, me.x), y = coord_of(g, 1, me.y), z = coord_of(g, 2, me.z);
-      int3 a, b;  // this warp's first and last point
-      a.x = __shfl_sync(0xffffffffu, me.x, 0), b.x = __shfl_sync(0xffffffffu, me.x, 31);
-      a.y = __shfl_sync(0xffffffffu, me.y, 0), b.y = __shfl_sync(0xffffffffu, me.y, 31);
-      a.z = __shfl_sync(0xffffffffu, me.z, 0), b.z = __shfl_sync(0xffffffffu, me.z, 31);
-      const PointBox mine = box_of(g, a, b);
       const bool live = w0 + lane <= last;
+      const float x = coord_of(g, 0, me.x), y = coord_of(g, 1, me.y), z = coord_of(g, 2, me.z);
       unsigned have = s_n[s][threadIdx.x];
-      for (int c0 = 0; c0 < kept; c0 += 32) {
-        const int c = c0 + lane;
-        unsigned m = __ballot_sync(0xffffffffu, c < kept && box_reached(mine, s_rec[min(c, kept - 1)], r2));
-        while (m) {
-          const int q = c0 + __ffs(m) - 1;
-          m &= m - 1;
-          if (live && dist2_rn(x, y, z, s_rec[q]) <= r2) have = hit(s, (int)s_idx[q], have);
+      int3 a;  // this warp's first point
+      a.x = __shfl_sync(0xffffffffu, me.x, 0);
+      a.y = __shfl_sync(0xffffffffu, me.y, 0);
+      if (__all_sync(0xffffffffu, live & (me.x == a.x) & (me.y == a.y))) {
+        const float lz = __shfl_sync(0xffffffffu, z, 0), hz = __shfl_sync(0xffffffffu, z, 31);
+        for (int c0 = 0; c0 < kept; c0 += 32) {
+          const int c = c0 + lane;
+          const float4 q = s_rec[min(c, kept - 1)];
+          const float dx = __fsub_rn(x, q.x), dy = __fsub_rn(y, q.y);
+          const float dxy = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+          const float dn = __fsub_rn(nearest_in(q.z, lz, hz), q.z);
+          unsigned m = __ballot_sync(0xffffffffu, c < kept && __fadd_rn(dxy, __fmul_rn(dn, dn)) <= r2);
+          while (m) {
+            const int b = __ffs(m) - 1;
+            m &= m - 1;
+            const float dz = __fsub_rn(z, __shfl_sync(0xffffffffu, q.z, b));
+            if (__fadd_rn(__shfl_sync(0xffffffffu, dxy, b), __fmul_rn(dz, dz)) <= r2) have = hit(s, (int)s_idx[c0 + b], have);
+          }
+        }
+      } else {
+        int3 e;  // and its last
+        a.z = __shfl_sync(0xffffffffu, me.z, 0);
+        e.x = __shfl_sync(0xffffffffu, me.x, 31);
+        e.y = __shfl_sync(0xffffffffu, me.y, 31);
+        e.z = __shfl_sync(0xffffffffu, me.z, 31);
+        const PointBox mine = box_of(g, a, e);
+        for (int c0 = 0; c0 < kept; c0 += 32) {
+          const int c = c0 + lane;
+          unsigned m = __ballot_sync(0xffffffffu, c < kept && box_reached(mine, s_rec[min(c, kept - 1)], r2));
+          while (m) {
+            const int q = c0 + __ffs(m) - 1;
+            m &= m - 1;
+            if (live && dist2_rn(x, y, z, s_rec[q]) <= r2) have = hit(s, (int)s_idx[q], have);
+          }
         }
       }
       s_n[s][threadIdx.x] = have;
+      // the point NB_THREADS further on
+      if (w0 + lane + NB_THREADS <= last) {
+        me.z += NB_THREADS;
+        if (me.z >= g.dim[2]) {
+          const int rows = me.z / g.dim[2];
+          me.z -= rows * g.dim[2];
+          me.y += rows;
+          if (me.y >= g.dim[1]) {
+            const int planes = me.y / g.dim[1];
+            me.y -= planes * g.dim[1];
+            me.x += planes;
+          }
+        }
+      } else {
+        me = index_of(g, last);
+      }
     }
     kept = 0;
     __syncthreads();  // the list is read
@@ -329,7 +390,7 @@ __device__ __forceinline__ void near_beads(const AttGridGeom& g, const float4* _
 
 // count + exclusive scan within each 1024 points; their totals to ws.  2500
 // beads, radius 5.2 A, 90.5 M points: 80.5 ms with every bead tested per point,
-// 1.04 ms now.
+// 0.97 ms now.
 __global__ void __launch_bounds__(NB_THREADS, 3)
 nb_count_kernel(AttGridGeom g, const float4* __restrict__ rec, int n_rec, float r2, uint2* __restrict__ hdr,
                 unsigned* __restrict__ ws, long long nvox) {
@@ -433,7 +494,7 @@ nb_add_kernel(uint2* __restrict__ hdr, const unsigned* __restrict__ ws, long lon
 }
 
 // The lists, in index order.  The same receptor and points: 120.7 ms with every
-// bead tested per point, 1.11 ms now.
+// bead tested per point, 1.04 ms now.
 __global__ void __launch_bounds__(NB_THREADS, 3)
 nb_fill_kernel(AttGridGeom g, const float4* __restrict__ rec, int n_rec, float r2, const uint2* __restrict__ hdr,
                uint16_t* __restrict__ list, long long nvox) {
