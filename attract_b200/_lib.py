@@ -99,6 +99,8 @@ SIGNATURES = {
     "att_kernel_status": (I, [C.POINTER(C.c_int), I, P]),
     "att_nbgrid_count_noalloc": (I, [C.POINTER(AttGridGeom), P, I, F, P, P, P]),
     "att_nbgrid_pack_records": (I, [P, P, LL, I, P, P]),
+    "att_nbgrid_quantile_workspace_bytes": (LL, [LL]),
+    "att_nbgrid_count_quantile": (I, [P, LL, F, LL, P, P, LL, P]),
     "att_kernel_debug_info": (I, [C.POINTER(C.c_ulonglong), I, P]),
     "att_allpairs_energy": (I, [P, I, P, I, P, I, I, P, I, I, F, P, P, P]),
     "att_minimise_schema": (I, [C.POINTER(AttGrid), I, C.POINTER(AttLigands), P, I, P, I, I, P, P, P,

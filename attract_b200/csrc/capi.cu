@@ -21,6 +21,9 @@ cudaError_t launch_nb_count(const AttGridGeom& g, const float* rec, int n_rec, f
                             unsigned long long* total, void* ws, cudaStream_t st);
 cudaError_t launch_nb_fill(const AttGridGeom& g, const float* rec, int n_rec, float radius, const uint32_t* hdr,
                            uint16_t* list, cudaStream_t st);
+long long nb_quantile_workspace_bytes(long long nvox);
+cudaError_t launch_nb_quantile(const uint32_t* hdr, long long nvox, float q, long long first, float* out, void* ws,
+                               cudaStream_t st);
 cudaError_t launch_repack(const AttGridGeom& g, const float* inner, const float* outer, void* bricks,
                           cudaStream_t st);
 cudaError_t launch_nb_pack(const uint32_t* hdr, const uint16_t* list, long long nvox, int rec_bytes, void* out,
@@ -443,6 +446,24 @@ extern "C" int att_nbgrid_pack_records(const uint32_t* hdr_dev, const uint16_t* 
   if (n_voxels == 0) return ATT_OK;
   cudaError_t e = launch_nb_pack(hdr_dev, list_dev, n_voxels, rec_bytes, records_dev, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "att_nbgrid_pack_records");
+  return ATT_OK;
+}
+
+extern "C" long long att_nbgrid_quantile_workspace_bytes(long long n_voxels) {
+  return n_voxels < 0 ? -1 : nb_quantile_workspace_bytes(n_voxels);
+}
+
+extern "C" int att_nbgrid_count_quantile(const uint32_t* hdr_dev, long long n_voxels, float q, long long first,
+                                         float* out_dev, void* workspace_dev, long long workspace_bytes, void* stream) {
+  REQUIRE(n_voxels >= 1, "n_voxels < 1");
+  REQUIRE(q >= 0.f && q <= 1.f, "q must be in [0, 1]");
+  REQUIRE(first >= 1 && first <= (1LL << 24), "first must be in [1, 2^24]");
+  REQUIRE(hdr_dev != nullptr && out_dev != nullptr && workspace_dev != nullptr, "hdr / out / workspace NULL");
+  REQUIRE(aligned(hdr_dev, 8) && aligned(out_dev, 4) && aligned(workspace_dev, 8), "hdr and workspace 8-B alignment");
+  REQUIRE(workspace_bytes >= nb_quantile_workspace_bytes(n_voxels), "workspace of %lld bytes < %lld", workspace_bytes,
+          nb_quantile_workspace_bytes(n_voxels));
+  cudaError_t e = launch_nb_quantile(hdr_dev, n_voxels, q, first, out_dev, workspace_dev, (cudaStream_t)stream);
+  if (e != cudaSuccess) return cuda_fail(e, "att_nbgrid_count_quantile");
   return ATT_OK;
 }
 

@@ -182,10 +182,8 @@ class Grid:
         """Fixed-size neighbour records (copied with the brick per bead and step): the
         smallest of 32/64/128 bytes whose inline entries hold 99 % of the
         non-empty lists; longer lists continue in the CSR list."""
-        counts = self.nb_hdr[:, 1]
         if rec_bytes is None:
-            nz = counts[counts > 0].to(torch.float32)
-            q = float(torch.quantile(nz[: 1 << 24], 0.99).item()) if nz.numel() else 0.0
+            q = list_length_quantile(self.nb_hdr, 0.99)
             rec_bytes = next((b for b in (32, 64, 128) if (b - 6) // 2 >= q), 128)
         self.nb_rec_bytes = rec_bytes
         self.nb_rec = torch.empty(self.nb_geom.n_voxels * rec_bytes, dtype=torch.uint8, device=self.device)
@@ -375,6 +373,21 @@ class Grid:
                     vals[ok] = self.rec_perm[vals[ok]]
                     lst[s0:s0 + n] = np.sort(vals)
         return f(self.inner), f(self.outer), hdr, lst
+
+
+def list_length_quantile(nb_hdr: torch.Tensor, q: float, first: int = 1 << 24) -> float:
+    """The ``q``-quantile of the first ``first`` non-zero counts of ``nb_hdr`` [points, 2]
+    (what ``torch.quantile`` gives for them; 0 when there are none)."""
+    lib = _lib.load()
+    n = nb_hdr.shape[0]
+    wsb = lib.att_nbgrid_quantile_workspace_bytes(n)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=nb_hdr.device)
+    out = torch.empty(1, dtype=torch.float32, device=nb_hdr.device)
+    with torch.cuda.device(nb_hdr.device):
+        st = torch.cuda.current_stream(nb_hdr.device).cuda_stream
+        _lib.check(lib.att_nbgrid_count_quantile(_lib.ptr(nb_hdr), n, float(q), first, _lib.ptr(out), _lib.ptr(ws),
+                                                 wsb, st), "att_nbgrid_count_quantile")
+    return float(out.item())
 
 
 def check_list_total(n_entries: int) -> None:

@@ -291,6 +291,15 @@ int att_nbgrid_fill(const AttGridGeom* geom, const float* rec_dev, int n_rec, fl
 int att_nbgrid_pack_records(const uint32_t* hdr_dev, const uint16_t* list_dev, long long n_voxels,
                             int rec_bytes, void* records_dev, void* stream);
 
+/* The q-quantile (0..1, linear between the two nearest) of the first `first`
+   (at most 2^24) non-zero counts of hdr_dev in grid order, to out_dev[0]; 0 when
+   all are zero.  The record size of att_nbgrid_pack_records follows it: the
+   smallest that holds 99 % of the non-empty lists inline.  (No counterpart in
+   the reference.) */
+long long att_nbgrid_quantile_workspace_bytes(long long n_voxels);
+int att_nbgrid_count_quantile(const uint32_t* hdr_dev, long long n_voxels, float q, long long first,
+                              float* out_dev, void* workspace_dev, long long workspace_bytes, void* stream);
+
 /* att_nbgrid_count without a caller workspace.  No counterpart in the
    reference (its neighbour lists come from a KD-tree on the host).
    Some callers of this library cannot allocate device memory: a plugin that

@@ -70,3 +70,21 @@ def test_lists_and_records_at_block_edges(n_rec, dim, refine, radius):
         assert np.array_equal(rec[:, : 2 * inl].copy().view(np.uint16), want)
         assert np.array_equal(rec[:, 2 * inl: 2 * inl + 2].copy().view(np.uint16)[:, 0], hdr[:, 1])
         assert np.array_equal(rec[:, rb - 4:].copy().view(np.uint32)[:, 0], hdr[:, 0] + inl)
+
+
+@pytest.mark.parametrize("n,top,zero,first", [(1, 3, 0.0, 1 << 24), (5, 70, 0.5, 1 << 24), (1023, 2, 0.9, 1 << 24),
+                                              (1025, 300, 0.3, 1 << 24), (70_001, 14, 0.6, 1 << 24),
+                                              (70_001, 60, 0.2, 1000), (70_001, 65_000, 0.5, 20_000),
+                                              (3_000_000, 31, 0.9, 1 << 24), (4096, 5, 1.0, 1 << 24)])
+def test_list_length_quantile_is_torchs(n, top, zero, first):
+    from attract_b200.grid import list_length_quantile
+
+    rng = np.random.default_rng(n + top)
+    c = np.where(rng.random(n) < zero, 0, rng.integers(1, top + 1, n))
+    hdr = torch.tensor(np.stack([np.arange(n), c], 1), dtype=torch.int32, device="cuda")
+    nz = torch.tensor(c[c > 0][:first], dtype=torch.float32)
+    for q in (0.99, 0.5, 0.0, 1.0):
+        want = float(torch.quantile(nz, q)) if len(nz) else 0.0
+        got = list_length_quantile(hdr, q, first)
+        assert abs(got - want) <= 2.0 ** -22 * want  # the last step's rounding
+        assert [b for b in (13, 29, 61) if b >= got] == [b for b in (13, 29, 61) if b >= want]
