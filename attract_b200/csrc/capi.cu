@@ -12,6 +12,7 @@ cudaError_t kernel_status(int* out, int clear, cudaStream_t st);
 cudaError_t kernel_debug_info(unsigned long long* out3, int clear, cudaStream_t st);
 int beads_per_lane(int S, int max_beads);
 int mode_beads_per_lane(int mode, int S, int max_beads);
+bool split_poses(int mode, int S, int threads, int max_beads, int n_tiles);
 size_t score_smem_bytes(int K, int threads, int rec_slot);
 cudaError_t launch_build_potential(const AttGridGeom& g, const float* rec, int n_rec, const float* pair,
                                    int n_rtypes, int n_ltypes, float cutoff, int outer, float* out,
@@ -253,10 +254,11 @@ extern "C" int att_energrad(const AttGrid* grids, int n_grids, const AttLigands*
   p.grad = grad_dev;
   p.status = status_dev;
   if (n_tiles == 0) return ATT_OK;
-  const int wpb = threads / 32;
+  const int mode = cfg->pose_format == 1 ? MODE_EVAL_MAT : MODE_EVAL;
+  p.split = split_poses(mode, S, threads, p.max_beads, n_tiles) ? 1 : 0;
+  const int wpb = p.split ? 1 : threads / 32;  // poses that a block takes
   const int blocks = (n_tiles + wpb - 1) / wpb;
-  cudaError_t e = launch_score(p, cfg->pose_format == 1 ? MODE_EVAL_MAT : MODE_EVAL, S, K, blocks, threads,
-                               (cudaStream_t)stream);
+  cudaError_t e = launch_score(p, mode, S, K, blocks, threads, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "att_energrad launch");
   return ATT_OK;
 }
@@ -398,7 +400,8 @@ extern "C" int att_energrad_backward(const AttGrid* grids, int n_grids, const At
     p.n_dgrid_outer = (long long)g.n_types * g.dim2[0] * g.dim2[1] * g.dim2[2] * 4;
   }
   if (n_tiles == 0) return ATT_OK;
-  const int wpb = threads / 32;
+  p.split = split_poses(MODE_BWD, S, threads, p.max_beads, n_tiles) ? 1 : 0;
+  const int wpb = p.split ? 1 : threads / 32;  // poses that a block takes
   const int blocks = (n_tiles + wpb - 1) / wpb;
   cudaError_t e = launch_score(p, MODE_BWD, S, K, blocks, threads, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "att_energrad_backward launch");

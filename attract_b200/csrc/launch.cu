@@ -4,13 +4,13 @@
 
 namespace att {
 
-static const void* kernel_of(int mode, int S, int K, bool one_grid) {
+static const void* kernel_of(int mode, int S, int K, bool one_grid, bool chunked) {
   switch (mode) {
     case MODE_EVAL:
-    case MODE_EVAL_MAT: return score_part_kernel<0>(mode, S, K, one_grid);
-    case MODE_MIN: return score_part_kernel<1>(mode, S, K, one_grid);
-    case MODE_BWD: return score_part_kernel<2>(mode, S, K, one_grid);
-    case MODE_QUAT: return score_part_kernel<3>(mode, S, K, one_grid);
+    case MODE_EVAL_MAT: return score_part_kernel<0>(mode, S, K, one_grid, chunked);
+    case MODE_MIN: return score_part_kernel<1>(mode, S, K, one_grid, chunked);
+    case MODE_BWD: return score_part_kernel<2>(mode, S, K, one_grid, chunked);
+    case MODE_QUAT: return score_part_kernel<3>(mode, S, K, one_grid, chunked);
   }
   return nullptr;
 }
@@ -28,12 +28,23 @@ int beads_per_lane(int S, int max_beads) {
 // 2, 4 and 8 beads per lane) to cover the copies' latency.  32 lanes: 40 beads,
 // 20 000 poses 78 -> 69 us; 100 beads, 8000 poses 97 -> 65; 200 beads, 5000 poses
 // 191 -> 76; 301 beads, 3000 matrices 184 -> 64; the adjoint of 100 beads, 8000 poses
-// 129 -> 105.  With at most 8 warps of work per SM the chunks' latencies add up instead:
-// 301 beads, 300 poses 20 -> 30 us, 100 beads 9.2 -> 13.3, less than the 13.5 us that a
-// call takes on the host.  One rule for all sizes keeps a pose's energy the same to the bit
-// in any batch.
+// 129 -> 105.  (Few poses: split_poses.)  One rule for all sizes keeps a pose's energy
+// the same to the bit in any batch.
 int mode_beads_per_lane(int mode, int S, int max_beads) {
   return mode == MODE_MIN || mode == MODE_QUAT ? beads_per_lane(S, max_beads) : 1;
+}
+
+// Whether the four warps of a block share each pose, a quarter of its chunks each:
+// while the blocks are at most two waves of 148 x 6, where a warp's chunks one after
+// another are the launch's time.  Calls of energrad with 4x4 poses, one warp per pose against
+// four (about 17 us are the host's): 301 beads, 100 poses 36.9 -> 16.9 us, 880 43.0 -> 24.7, 1500
+// 50.4 -> 38.3; 160 beads, 880 poses 24.6 -> 18.5; 100 beads, 1500 poses 21.3 -> 20.5.
+// Beyond, whole poses per warp keep more warps busy: 100 beads, 2200 poses 24.6 -> 26.7;
+// two chunks leave two warps idle: 40 beads, 2200 poses 17.0 -> 20.5.  The sums are the
+// same to the bit.
+bool split_poses(int mode, int S, int threads, int max_beads, int n_tiles) {
+  if (mode == MODE_MIN || mode == MODE_QUAT || S != 32 || threads != 128 || max_beads <= 64) return false;
+  return n_tiles <= 148 * 6 * 2;
 }
 
 size_t score_smem_bytes(int K, int threads, int rec_slot) {
@@ -56,7 +67,7 @@ static cudaError_t allow_smem(const void* k, size_t bytes) {
 
 static cudaError_t launch_one(const KParams& p, int mode, int S, int K, bool one_grid, int blocks, int threads,
                               cudaStream_t st) {
-  const void* k = kernel_of(mode, S, K, one_grid);
+  const void* k = kernel_of(mode, S, K, one_grid, p.max_beads > S * K);
   if (k == nullptr) return cudaErrorInvalidValue;
   const size_t smem = mode_smem_bytes(mode, K, threads, p.rec_slot);
   cudaError_t e = allow_smem(k, smem);
@@ -111,7 +122,7 @@ cudaError_t kernel_debug_info(unsigned long long* out3, int clear, cudaStream_t 
 }
 
 cudaError_t occupancy_blocks(int mode, int S, int K, int threads, int rec_slot, bool one_grid, int* blocks_per_sm) {
-  const void* k = kernel_of(mode, S, K, one_grid);
+  const void* k = kernel_of(mode, S, K, one_grid, true);  // (the minimisers')
   if (k == nullptr) return cudaErrorInvalidValue;
   const size_t smem = mode_smem_bytes(mode, K, threads, rec_slot);
   const cudaError_t e = allow_smem(k, smem);

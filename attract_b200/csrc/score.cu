@@ -181,6 +181,51 @@ __device__ __forceinline__ void team_sum6(float& a0, float& a1, float& a2, float
   a5 = __shfl_sync(F, r, lead + H1 + H3);
 }
 
+// The same for N = 6 or 12 values, the sums left where they are (12: one level of
+// halving more; 13 / 12 shuffles at S = 32 / 16, where xor trees take 60 / 48): the first of team
+// lanes scatter_lane(i) and its neighbour hold sum i.  A value's additions are those of
+// the xor tree, in its order: the same bits.  With one bead per lane: quaternion protocol, 24
+// beads, 20 000 poses 9.57 -> 9.32 ms; energrad of 65 536 24-bead 4x4 poses 139.0 ->
+// 131.5 us.  (The Euler minimisers keep team_sum6: 25.3 ms against 25.0 with this.)
+template <int N, int S>
+__host__ __device__ constexpr int scatter_lane(int i) {
+  return N == 12 ? (i / 6 * (S / 2) + i % 6 / 3 * (S / 4) + (i % 3 == 0 ? 0 : i % 3 == 1 ? S / 8 : S / 16))
+                 : (i / 3 * (S / 2) + (i % 3 == 0 ? 0 : i % 3 == 1 ? S / 4 : S / 8));
+}
+template <int N, int S>
+__device__ __forceinline__ float team_scatter(float (&a)[N], int lane) {
+  constexpr unsigned F = 0xffffffffu;
+  static_assert((N == 6 && S >= 8) || (N == 12 && S >= 16), "a level per halving");
+  float k[N / 2];  // kept: the first or the second half
+  const bool h1 = lane & (S / 2);
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    k[i] = h1 ? a[N / 2 + i] : a[i];
+    k[i] += __shfl_xor_sync(F, h1 ? a[i] : a[N / 2 + i], S / 2);
+  }
+  int off = S / 4;
+  if (N == 12) {
+    const bool h = lane & off;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float send = h ? k[i] : k[i + N / 2 - 3];
+      k[i] = h ? k[i + N / 2 - 3] : k[i];
+      k[i] += __shfl_xor_sync(F, send, off);
+    }
+    off >>= 1;
+  }
+  const bool h2 = lane & off, h3 = lane & (off >> 1);
+  float m = h2 ? k[1] : k[0];  // kept: the first or the second of three
+  m += __shfl_xor_sync(F, h2 ? k[0] : k[1], off);
+  k[2] += __shfl_xor_sync(F, k[2], off);
+  off >>= 1;
+  float r = h3 ? k[2] : m;     // kept: that one, or the third
+  r += __shfl_xor_sync(F, h3 ? m : k[2], off);
+#pragma unroll
+  for (off >>= 1; off >= 1; off >>= 1) r += __shfl_xor_sync(F, r, off);
+  return r;
+}
+
 __device__ __forceinline__ int find_segment(const KParams& p, int tile) {
   int lo = 0, hi = p.n_segs - 1;
   while (lo < hi) {
@@ -240,7 +285,8 @@ __device__ __forceinline__ void pair_term_masked(const KParams& p, const KGrid& 
 template <int S, int K>
 __host__ __device__ constexpr int score_blocks_per_sm() { return K == 1 ? (S == 32 ? 6 : 5) : K == 2 ? 4 : 2; }
 
-template <int S, int K, int MODE, bool ONE>
+// CHUNKED: ligands may have more beads than a team's slots.
+template <int S, int K, int MODE, bool ONE, bool CHUNKED>
 __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kernel(const __grid_constant__ KParams p) {
   constexpr int P = 32 / S;      // poses per warp
   constexpr int NB = S * K;      // bead slots per pose
@@ -265,6 +311,12 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
   constexpr int ARM_BYTES = ACC9 ? 16 : 0;
   uint32_t* pbuf = reinterpret_cast<uint32_t*>(nrec + 32 * K * (RS + 16 + ARM_BYTES));
   const int tbase = slot * NB;  // this team's first bead record
+  // Single evaluations of 32 lanes sum a ligand of more than two chunks in four classes
+  // (chunk mod 4) and the classes in order, in one warp or (p.split) with the block's
+  // four warps on one pose, a class each: the same sums either way.  (The classes' own
+  // sums cost a warp 1 % of 301 beads, 3 % of 100; two chunks are summed as one class.)
+  constexpr bool CLASSES = CHUNKED && S == 32 && MODE != MODE_MIN && !QUAT;
+  const bool split = CLASSES && p.split != 0;
   // the pair loop and phase D are compiled per gradient mode; with several beads
   // per lane the kernels over several grids hold the reference mode only (launch_score)
   const bool ref_grad = (!ONE && K > 1) || p.grad_mode == ATT_GRAD_REFERENCE;
@@ -304,7 +356,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
     if (lane == 0) t0 = atomicAdd(p.counter, 1);
     tile = __shfl_sync(0xffffffffu, t0, 0);
   } else {
-    tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    tile = split ? (int)blockIdx.x : (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   }
 
   auto next_tile = [&]() {
@@ -313,7 +365,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
       if (lane == 0) t0 = atomicAdd(p.counter, 1);
       tile = __shfl_sync(0xffffffffu, t0, 0);
     } else {
-      tile += nwarps;
+      tile += split ? (int)gridDim.x : nwarps;
     }
   };
 
@@ -360,7 +412,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
     // NB beads; the chunk count is warp-uniform (the chunk loop holds warp
     // barriers and shuffles)
     const int nchunk = __reduce_max_sync(0xffffffffu, (unsigned)((Ntot + NB - 1) / NB));
-    const bool multi = nchunk > 1;
+    const bool multi = CHUNKED && nchunk > 1;
 
     // owned ligand beads (ligand frame), resident for the whole tile
     float lx[K], ly[K], lz[K];
@@ -519,7 +571,14 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 #pragma unroll
       for (int k = 0; k < (ACC9 ? 9 : 3); ++k) acc_t[k] = 0.f;
 
-      for (int chunk = 0; chunk < nchunk; ++chunk) {
+      constexpr bool SCATTER = K == 1 && (ACC9 ? S >= 16 : CLASSES);
+      constexpr int NS = ACC9 ? 12 : 6;  // forces and torques
+      float my_sum = 0.f;  // SCATTER: the sum that this lane holds
+      float my_tot = 0.f;  // CLASSES, several chunks: that, over the classes
+      const bool classes = CLASSES && nchunk > 2;
+      const int cls_end = classes ? min(nchunk, 4) : 1;
+      for (int cls = split ? warp : 0; cls < cls_end; cls += split ? 4 : 1) {
+      for (int chunk = cls; chunk < (CHUNKED ? nchunk : 1); chunk += classes ? 4 : 1) {
       const int c0 = chunk * NB;
       const int N = max(0, min(Ntot - c0, NB));  // beads of this chunk
       if (multi) load_beads(c0);
@@ -648,8 +707,10 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
       // of one brick or record, so that a copy instruction fills whole 128-byte
       // lines instead of one chunk of 32 lines; each lane waits for its own
       // copies, and the warp barrier after the wait hands every slot to its
-      // owner.  (Listing in the minimisers costs them registers and spills:
-      // 14 % slower on 18-30-bead ligands; one chunk of 32 lines per instruction costs
+      // owner: the bricks before phase D, the records after it (energrad of 65 536
+      // 24-bead poses 129.4 -> 127.9 us; 126.8 with a kernel for ligands of one chunk, CHUNKED
+      // false; the adjoint, whose phase C is first, waits for both at once).
+      // (Listing in the minimisers costs them registers and spills: 14 % slower on 18-30-bead ligands; one chunk of 32 lines per instruction costs
       // the single-evaluation modes a factor 1.9.)  The grid is warp-uniform:
       // a warp's teams share one segment.
       if constexpr (MODE == MODE_MIN || QUAT) {
@@ -721,6 +782,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
             const unsigned c = (i & 7u) * 16u;
             cp16(smem_u32(bricks) + e.y * 128u + c, gb + ((size_t)e.x * 128u + c));
           }
+          if (MODE != MODE_BWD) cp_commit();  // group 1: the bricks
           if (nv_cp != 0u) {
             const unsigned RB = (unsigned)G.nb_rec_bytes;  // 32, 64 or 128
             const int rsh = __ffs(RB) - 5;                 // log2 of the 16-byte chunks per record
@@ -730,7 +792,12 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
               cp16(smem_u32(nrec) + e.y * (unsigned)RS + c, G.nb_rec + ((size_t)e.x * RB + c));
             }
           }
-          cp_commit_wait();
+          if (MODE != MODE_BWD) {
+            cp_commit();  // group 2: the records (phase C waits for it, after phase D)
+            cp_wait<1>();
+          } else {
+            cp_commit_wait();
+          }
           __syncwarp();
         }
       }
@@ -828,7 +895,12 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
       // 0.496 ms with phase D first; the forward modes gain 2 % with it first).
       if constexpr (MODE != MODE_BWD) run_d();
       // the minimisers: this lane's records have landed
-      if constexpr (MODE == MODE_MIN || QUAT) cp_wait<0>();
+      if constexpr (MODE == MODE_MIN || QUAT) {
+        cp_wait<0>();
+      } else if constexpr (MODE != MODE_BWD) {  // every lane's records
+        cp_wait<0>();
+        __syncwarp();
+      }
       auto phase_c = [&]() {
 
       // ---------------- phase C: neighbour pairs, balanced over the team.
@@ -1003,9 +1075,25 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
       __syncwarp();
       }  // chunks
 
-      // ---------------- team reduction and output / ADAM
+      // ---------------- team reduction
       if (need_e) acc_e = team_sum<S>(acc_e);
-      if constexpr (!ACC9 && (K == 1 || S == 32)) {
+      if constexpr (SCATTER) {
+        float v[NS];
+        v[0] = acc_gx;
+        v[1] = acc_gy;
+        v[2] = acc_gz;
+#pragma unroll
+        for (int k = 0; k < NS - 3; ++k) v[3 + k] = acc_t[k];
+        my_sum = team_scatter<NS, S>(v, lane);
+        if constexpr (CLASSES) {
+          if (multi) {  // odd lanes, whose neighbours hold their sums too, carry the energy
+            my_tot += (lane & 1) ? acc_e : my_sum;
+            acc_e = acc_gx = acc_gy = acc_gz = 0.f;
+#pragma unroll
+            for (int k = 0; k < (ACC9 ? 9 : 3); ++k) acc_t[k] = 0.f;
+          }
+        }
+      } else if constexpr (!ACC9 && (K == 1 || S == 32)) {
         team_sum6<S>(acc_gx, acc_gy, acc_gz, acc_t[0], acc_t[1], acc_t[2], lane);
       } else {
         acc_gx = team_sum<S>(acc_gx);
@@ -1014,6 +1102,33 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 #pragma unroll
         for (int k = 0; k < (ACC9 ? 9 : 3); ++k) acc_t[k] = team_sum<S>(acc_t[k]);
       }
+      }  // classes
+      if constexpr (CLASSES) {
+        if (multi) {
+          if (split) {  // (block-uniform: the block's warps have one tile)
+            // the warps' sums through their pair buffers, which nothing reads now
+            reinterpret_cast<float*>(pbuf)[lane] = my_tot;
+            __syncthreads();
+            if (warp == 0) {
+              const size_t next = warp_smem_bytes(K, p.rec_slot, ACC9) / 4;
+              for (int w = 1; w < cls_end; ++w) my_tot += reinterpret_cast<const float*>(pbuf)[lane + w * next];
+            }
+            __syncthreads();
+          }
+          my_sum = my_tot;
+          acc_e = __shfl_sync(0xffffffffu, my_tot, 1);
+        }
+        if (split && warp != 0) valid = false;  // the first warp writes
+      }
+      if constexpr (SCATTER) {
+        acc_gx = __shfl_sync(0xffffffffu, my_sum, lead + scatter_lane<NS, S>(0));
+        acc_gy = __shfl_sync(0xffffffffu, my_sum, lead + scatter_lane<NS, S>(1));
+        acc_gz = __shfl_sync(0xffffffffu, my_sum, lead + scatter_lane<NS, S>(2));
+#pragma unroll
+        for (int k = 0; k < NS - 3; ++k) acc_t[k] = __shfl_sync(0xffffffffu, my_sum, lead + scatter_lane<NS, S>(3 + k));
+      }
+
+      // ---------------- output / ADAM
       if (!ACC9) {  // torque about the pose's translation: sum X x g - t x sum g
         acc_t[0] -= fmaf(ty, acc_gz, -tz * acc_gy);
         acc_t[1] -= fmaf(tz, acc_gx, -tx * acc_gz);
@@ -1172,9 +1287,11 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 // this part's (S, K) instantiations and error words
 // ---------------------------------------------------------------------------
 template <int MODE, bool ONE>
-static const void* kernel_of_shape(int S, int K) {
+static const void* kernel_of_shape(int S, int K, bool chunked) {
 #define ATT_CASE(s_, k_) \
-  if (S == s_ && K == k_) return (const void*)score_kernel<s_, k_, MODE, ONE>;
+  if (S == s_ && K == k_) return (const void*)score_kernel<s_, k_, MODE, ONE, true>;
+  if constexpr (MODE != MODE_MIN && MODE != MODE_QUAT)
+    if (S == 32 && !chunked) return (const void*)score_kernel<32, 1, MODE, ONE, false>;
   ATT_CASE(32, 1) ATT_CASE(16, 1) ATT_CASE(8, 1)
   if constexpr (MODE == MODE_MIN || MODE == MODE_QUAT) {  // (mode_beads_per_lane)
     ATT_CASE(32, 2) ATT_CASE(32, 4) ATT_CASE(32, 8)
@@ -1186,9 +1303,9 @@ static const void* kernel_of_shape(int S, int K) {
 }
 
 template <>
-const void* score_part_kernel<ATT_SCORE_PART>(int mode, int S, int K, bool one_grid) {
+const void* score_part_kernel<ATT_SCORE_PART>(int mode, int S, int K, bool one_grid, bool chunked) {
 #define ATT_MODE(m_) \
-  if (mode == m_) return one_grid ? kernel_of_shape<m_, true>(S, K) : kernel_of_shape<m_, false>(S, K);
+  if (mode == m_) return one_grid ? kernel_of_shape<m_, true>(S, K, chunked) : kernel_of_shape<m_, false>(S, K, chunked);
 #if ATT_SCORE_PART == 0
   ATT_MODE(MODE_EVAL) ATT_MODE(MODE_EVAL_MAT)
 #elif ATT_SCORE_PART == 1

@@ -8,12 +8,14 @@ namespace att {
 
 constexpr int SCORE_PARTS = 4;  // 0: the single evaluations, 1: MODE_MIN, 2: MODE_BWD, 3: MODE_QUAT
 
-// the kernel of (mode, lanes per pose, beads per lane), or NULL when the part does not hold the mode
-template <int PART> const void* score_part_kernel(int mode, int S, int K, bool one_grid);
+// the kernel of (mode, lanes per pose, beads per lane), or NULL when the part does not hold the
+// mode; chunked: a ligand may have more beads than the team's slots (single evaluations
+// of 32 lanes; the other kernels take any)
+template <int PART> const void* score_part_kernel(int mode, int S, int K, bool one_grid, bool chunked);
 template <int PART> cudaError_t score_part_status(int* out, int clear, cudaStream_t st);
 template <int PART> cudaError_t score_part_debug(unsigned long long* out3, int clear, cudaStream_t st);
 #define ATT_DECLARE_PART(i_) \
-  template <> const void* score_part_kernel<i_>(int, int, int, bool); \
+  template <> const void* score_part_kernel<i_>(int, int, int, bool, bool); \
   template <> cudaError_t score_part_status<i_>(int*, int, cudaStream_t); \
   template <> cudaError_t score_part_debug<i_>(unsigned long long*, int, cudaStream_t);
 ATT_DECLARE_PART(0) ATT_DECLARE_PART(1) ATT_DECLARE_PART(2) ATT_DECLARE_PART(3)
