@@ -433,11 +433,14 @@ nb_count_kernel(AttGridGeom g, const float4* __restrict__ rec, int n_rec, float 
   }
 }
 
-// exclusive scan of the block totals (one block, 8 consecutive words per thread and step)
+// exclusive scan of the block totals (one block, 8 consecutive words per thread and step).
+// A word holds 1024 points' entries (at most 1024 x 65 534), so a thread's eight fit in 32
+// bits; a step's 8192 words do not (from 512 entries per point on), and the total has to be true
+// for the host to refuse lists beyond 32-bit starts: 64 bits from the warp's scan on.
 constexpr int SCAN_ITEMS = 8;
 __global__ void __launch_bounds__(SCAN_THREADS)
 nb_scan_blocks_kernel(unsigned* __restrict__ ws, int nblk, unsigned long long* __restrict__ total) {
-  __shared__ unsigned wsum[SCAN_THREADS / 32];
+  __shared__ unsigned long long wsum[SCAN_THREADS / 32];
   __shared__ unsigned long long carry;
   if (threadIdx.x == 0) carry = 0ull;
   __syncthreads();
@@ -450,26 +453,26 @@ nb_scan_blocks_kernel(unsigned* __restrict__ ws, int nblk, unsigned long long* _
       v[k] = i0 + k < nblk ? ws[i0 + k] : 0u;
       c += v[k];
     }
-    unsigned inc = c;
+    unsigned long long inc = c;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      const unsigned t = __shfl_up_sync(0xffffffffu, inc, off);
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, off);
       if (lane >= off) inc += t;
     }
     if (lane == 31) wsum[w] = inc;
     __syncthreads();
     if (w == 0) {
-      unsigned s = wsum[lane];
+      unsigned long long s = wsum[lane];
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
-        const unsigned t = __shfl_up_sync(0xffffffffu, s, off);
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, s, off);
         if (lane >= off) s += t;
       }
       wsum[lane] = s;
     }
     __syncthreads();
     const unsigned long long cb = carry;
-    unsigned before = (unsigned)(cb + (w > 0 ? wsum[w - 1] : 0u) + inc - c);
+    unsigned before = (unsigned)(cb + (w > 0 ? wsum[w - 1] : 0ull) + inc - c);
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
       if (i0 + k < nblk) ws[i0 + k] = before;
