@@ -47,7 +47,7 @@ struct KParams {
   const int* seg_tile;
   int n_segs, n_tiles;
   int n_grids, n_lig, max_beads;  // bounds of the segment / conformer / bead-range checks
-  int split;                      // single evaluations of 32 lanes: a pose's chunks over the block's warps
+  int split;                      // single evaluations: a tile's chunks over the block's warps
   int grid_sel;                   // kernels over one grid: the segments' index of grid[0]
   int n_pose_rows;
   const float* pose_in;

@@ -24,27 +24,32 @@ int beads_per_lane(int S, int max_beads) {
 
 // A minimiser keeps every bead's brick and record in shared memory from step to
 // step, so its lanes hold all of a ligand's beads.  A single evaluation copies each
-// once whatever its chunk: one bead per lane leaves room for 24 warps per SM (16, 8 and 4 at
-// 2, 4 and 8 beads per lane) to cover the copies' latency.  32 lanes: 40 beads,
+// once whatever its chunk: one bead per lane leaves room for 24 warps per SM at 32 lanes, 20 at
+// 8 and 16 (5 blocks; at 32 lanes too with 128-byte records) where 2, 4 and 8 beads per lane
+// left 16, 8 and 4, to cover the copies' latency.  energrad, before and now: 32 lanes: 40 beads,
 // 20 000 poses 78 -> 69 us; 100 beads, 8000 poses 97 -> 65; 200 beads, 5000 poses
 // 191 -> 76; 301 beads, 3000 matrices 184 -> 64; the adjoint of 100 beads, 8000 poses
-// 129 -> 105.  (Few poses: split_poses.)  One rule for all sizes keeps a pose's energy
-// the same to the bit in any batch.
+// 129 -> 105.  16 lanes, 30 000 poses: 24 beads 91 -> 60 us, 60 beads 224 -> 112; 8 lanes: 24 beads
+// 108 -> 55, 60 beads 345 -> 116, 100 beads 503 -> 175.  (Few poses: split_poses.)  One rule for all
+// sizes keeps a pose's energy the same to the bit in any batch.
 int mode_beads_per_lane(int mode, int S, int max_beads) {
   return mode == MODE_MIN || mode == MODE_QUAT ? beads_per_lane(S, max_beads) : 1;
 }
 
-// Whether the four warps of a block share each pose, a quarter of its chunks each:
-// while the blocks are at most two waves of 148 x 6, where a warp's chunks one after
-// another are the launch's time.  Calls of energrad with 4x4 poses, one warp per pose against
-// four (about 17 us are the host's): 301 beads, 100 poses 36.9 -> 16.9 us, 880 43.0 -> 24.7, 1500
-// 50.4 -> 38.3; 160 beads, 880 poses 24.6 -> 18.5; 100 beads, 1500 poses 21.3 -> 20.5.
-// Beyond, whole poses per warp keep more warps busy: 100 beads, 2200 poses 24.6 -> 26.7;
-// two chunks leave two warps idle: 40 beads, 2200 poses 17.0 -> 20.5.  The sums are the
-// same to the bit.
+// Whether the four warps of a block share each tile of poses, a quarter of the chunks each:
+// from three chunks on, while the blocks are at most two waves (6 blocks per SM at 32 lanes, 5 at 8 and
+// 16), where a warp's chunks one after another are the launch's time.  energrad, one warp per
+// tile against four, without the host's time: 32 lanes: 301 beads, 300 poses 34.3 -> 14.4 us, 1500
+// 44.7 -> 36.7, 3000 60.2 -> 62.2; 100 beads, 300 poses 15.8 -> 7.8, 2000 22.8 -> 22.1.  16 lanes (two poses
+// per tile): 100 beads, 600 poses 25.7 -> 11.6, 2400 28.7 -> 24.8, 3000 32.1 -> 31.6; 40 beads, 3000 16.7 -> 18.6.
+// 8 lanes (four poses): 40 beads, 1200 poses 21.0 -> 11.5, 4800 23.9 -> 24.0, 6000 26.5 -> 29.5; 301 beads,
+// 1200 130 -> 42.  Two chunks leave two warps idle (32 lanes: 40 beads, 2200 poses 17.0 -> 20.5).
+// The sums are the same to the bit.
 bool split_poses(int mode, int S, int threads, int max_beads, int n_tiles) {
-  if (mode == MODE_MIN || mode == MODE_QUAT || S != 32 || threads != 128 || max_beads <= 64) return false;
-  return n_tiles <= 148 * 6 * 2;
+  if (mode == MODE_MIN || mode == MODE_QUAT || threads != 128 || max_beads <= 2 * S) return false;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return n_tiles <= sms * (S == 32 ? 6 : 5) * 2;
 }
 
 size_t score_smem_bytes(int K, int threads, int rec_slot) {

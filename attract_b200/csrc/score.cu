@@ -311,11 +311,11 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
   constexpr int ARM_BYTES = ACC9 ? 16 : 0;
   uint32_t* pbuf = reinterpret_cast<uint32_t*>(nrec + 32 * K * (RS + 16 + ARM_BYTES));
   const int tbase = slot * NB;  // this team's first bead record
-  // Single evaluations of 32 lanes sum a ligand of more than two chunks in four classes
+  // Single evaluations sum a ligand of more than two chunks in four classes
   // (chunk mod 4) and the classes in order, in one warp or (p.split) with the block's
   // four warps on one pose, a class each: the same sums either way.  (The classes' own
   // sums cost a warp 1 % of 301 beads, 3 % of 100; two chunks are summed as one class.)
-  constexpr bool CLASSES = CHUNKED && S == 32 && MODE != MODE_MIN && !QUAT;
+  constexpr bool CLASSES = CHUNKED && MODE != MODE_MIN && !QUAT;
   const bool split = CLASSES && p.split != 0;
   // the pair loop and phase D are compiled per gradient mode; with several beads
   // per lane the kernels over several grids hold the reference mode only (launch_score)
@@ -573,8 +573,14 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 
       constexpr bool SCATTER = K == 1 && (ACC9 ? S >= 16 : CLASSES);
       constexpr int NS = ACC9 ? 12 : 6;  // forces and torques
+      // whether the sums' lanes come in pairs that hold the same: odd ones can carry the energy
+      constexpr bool PAIRED = SCATTER && S >= (ACC9 ? 32 : 16);
       float my_sum = 0.f;  // SCATTER: the sum that this lane holds
       float my_tot = 0.f;  // CLASSES, several chunks: that, over the classes
+      float e_tot = 0.f;   //   the energy, where no lane is free for it
+      float all_tot[CLASSES && !SCATTER ? NS : 1];  // and all sums, without a scatter
+#pragma unroll
+      for (int k = 0; k < (CLASSES && !SCATTER ? NS : 1); ++k) all_tot[k] = 0.f;
       const bool classes = CLASSES && nchunk > 2;
       const int cls_end = classes ? min(nchunk, 4) : 1;
       for (int cls = split ? warp : 0; cls < cls_end; cls += split ? 4 : 1) {
@@ -1087,7 +1093,8 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
         my_sum = team_scatter<NS, S>(v, lane);
         if constexpr (CLASSES) {
           if (multi) {  // odd lanes, whose neighbours hold their sums too, carry the energy
-            my_tot += (lane & 1) ? acc_e : my_sum;
+            if constexpr (!PAIRED) e_tot += acc_e;
+            my_tot += PAIRED && (lane & 1) ? acc_e : my_sum;
             acc_e = acc_gx = acc_gy = acc_gz = 0.f;
 #pragma unroll
             for (int k = 0; k < (ACC9 ? 9 : 3); ++k) acc_t[k] = 0.f;
@@ -1101,22 +1108,62 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
         acc_gz = team_sum<S>(acc_gz);
 #pragma unroll
         for (int k = 0; k < (ACC9 ? 9 : 3); ++k) acc_t[k] = team_sum<S>(acc_t[k]);
+        if constexpr (CLASSES) {
+          if (multi) {
+            e_tot += acc_e;
+            all_tot[0] += acc_gx;
+            all_tot[1] += acc_gy;
+            all_tot[2] += acc_gz;
+            acc_e = acc_gx = acc_gy = acc_gz = 0.f;
+#pragma unroll
+            for (int k = 0; k < NS - 3; ++k) {
+              all_tot[3 + k] += acc_t[k];
+              acc_t[k] = 0.f;
+            }
+          }
+        }
       }
       }  // classes
       if constexpr (CLASSES) {
         if (multi) {
           if (split) {  // (block-uniform: the block's warps have one tile)
             // the warps' sums through their pair buffers, which nothing reads now
-            reinterpret_cast<float*>(pbuf)[lane] = my_tot;
+            float* mine = reinterpret_cast<float*>(pbuf);
+            const size_t next = warp_smem_bytes(K, p.rec_slot, ACC9) / 4;
+            if constexpr (SCATTER) {
+              mine[lane] = my_tot;
+              if constexpr (!PAIRED) mine[32 + lane] = e_tot;
+            } else if (tl == 0) {  // a team's sums are on all of its lanes
+#pragma unroll
+              for (int k = 0; k < NS; ++k) mine[slot * (NS + 1) + k] = all_tot[k];
+              mine[slot * (NS + 1) + NS] = e_tot;
+            }
             __syncthreads();
             if (warp == 0) {
-              const size_t next = warp_smem_bytes(K, p.rec_slot, ACC9) / 4;
-              for (int w = 1; w < cls_end; ++w) my_tot += reinterpret_cast<const float*>(pbuf)[lane + w * next];
+              for (int w = 1; w < cls_end; ++w) {
+                const float* theirs = mine + w * next;
+                if constexpr (SCATTER) {
+                  my_tot += theirs[lane];
+                  if constexpr (!PAIRED) e_tot += theirs[32 + lane];
+                } else {
+#pragma unroll
+                  for (int k = 0; k < NS; ++k) all_tot[k] += theirs[slot * (NS + 1) + k];
+                  e_tot += theirs[slot * (NS + 1) + NS];
+                }
+              }
             }
             __syncthreads();
           }
-          my_sum = my_tot;
-          acc_e = __shfl_sync(0xffffffffu, my_tot, 1);
+          if constexpr (SCATTER) {
+            my_sum = my_tot;
+          } else {
+            acc_gx = all_tot[0];
+            acc_gy = all_tot[1];
+            acc_gz = all_tot[2];
+#pragma unroll
+            for (int k = 0; k < NS - 3; ++k) acc_t[k] = all_tot[3 + k];
+          }
+          acc_e = PAIRED ? __shfl_sync(0xffffffffu, my_tot, lead + 1) : e_tot;
         }
         if (split && warp != 0) valid = false;  // the first warp writes
       }
