@@ -59,9 +59,12 @@ namespace att {
 // reads and clears the words of all parts
 static __device__ int g_kernel_error = 0;
 
-// Debug builds (-DATT_BOUNDS_CHECK) check every computed index against its
-// buffer before the access, skip the access when it is out of range, and
-// record the first failure (check code, index, bound) for att_kernel_debug_info.
+// Debug builds (-DATT_BOUNDS_CHECK) check every address that the kernels form --
+// brick, record, list and receptor indices, pair rows, bead slots, pair-buffer words and copy
+// lists against their buffers, shared-memory addresses against the block's dynamic
+// shared memory, the descriptors' pointers and 16-byte accesses for alignment -- before the
+// access, skip the access when the check fails, and record the first failure (check
+// code, index, bound) for att_kernel_debug_info.
 static __device__ unsigned long long g_kernel_debug[3] = {0ull, 0ull, 0ull};
 #ifdef ATT_BOUNDS_CHECK
 static __device__ __noinline__ void bounds_report(int code, long long a, long long b) {
@@ -72,8 +75,18 @@ static __device__ __noinline__ void bounds_report(int code, long long a, long lo
   }
 }
 #define ATT_CHECK(cond, code, a, b) ((cond) ? true : (bounds_report((code), (a), (b)), false))
+// whether [addr, addr + bytes) lies in the block's dynamic shared memory, `bytes`-aligned
+static __device__ __forceinline__ bool dyn_smem_ok(uint32_t addr, uint32_t bytes) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  uint32_t n;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(n));
+  const uint32_t off = addr - (uint32_t)__cvta_generic_to_shared(smem_raw);
+  return (addr & (bytes - 1u)) == 0u && off < n && off + bytes <= n;
+}
+#define ATT_CHECK_SMEM(addr, bytes, code) ATT_CHECK(dyn_smem_ok((addr), (bytes)), (code), (addr), (bytes))
 #else
 #define ATT_CHECK(cond, code, a, b) true
+#define ATT_CHECK_SMEM(addr, bytes, code) true
 #endif
 
 // ---------------------------------------------------------------------------
@@ -89,7 +102,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // mbarrier: 3.8 % faster in the minimiser, per lane; 11 % faster for single
 // evaluations, spread over the warp.)
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
-  if (!ATT_CHECK(((dst | (uint32_t)(uintptr_t)src) & 15u) == 0u, 7, dst, (long long)(uintptr_t)src)) return;
+  if (!ATT_CHECK(((uintptr_t)src & 15u) == 0u, 7, dst, (long long)(uintptr_t)src)) return;
+  if (!ATT_CHECK_SMEM(dst, 16u, 8)) return;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ uint32_t lanemask_lt() {
@@ -115,19 +129,21 @@ __device__ __forceinline__ void cp_wait() {
 // fault).
 __device__ __forceinline__ unsigned lds_u16(const void* p) {
   unsigned short v;
+  if (!ATT_CHECK_SMEM(smem_u32(p), 2u, 9)) return 0u;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(smem_u32(p)) : "memory");
   return v;
 }
 
 __device__ __forceinline__ unsigned lds_u32(const void* p) {
   unsigned v;
+  if (!ATT_CHECK_SMEM(smem_u32(p), 4u, 10)) return 0u;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
   return v;
 }
 
 __device__ __forceinline__ uint4 lds_u128(const void* p) {  // p 16-byte aligned
   uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (!ATT_CHECK((smem_u32(p) & 15u) == 0u, 8, smem_u32(p), 0)) return v;
+  if (!ATT_CHECK_SMEM(smem_u32(p), 16u, 11)) return v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "r"(smem_u32(p)) : "memory");
   return v;
@@ -249,7 +265,8 @@ __device__ __forceinline__ void pair_term_masked(const KParams& p, const KGrid& 
   const float dsq = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
   const int rt = __float_as_int(r.w);
   const bool hit = (dsq < G.plateau2) & ((unsigned)rt < (unsigned)G.n_rtypes) & jok;
-  const int idx = hit ? bp.lt * G.n_rtypes + rt : 0;
+  int idx = hit ? bp.lt * G.n_rtypes + rt : 0;
+  if (!ATT_CHECK(idx >= 0 && idx < G.n_rtypes * G.n_ltypes, 12, idx, (long long)G.n_rtypes * G.n_ltypes)) idx = 0;
   float4 p0, p1;  // rc, ac, emin, rmin2 / ivor, eplat, gplat, rcap2: one 32-B row
   ldg_f4x2(G.pair + (size_t)(unsigned)idx * 2, p0, p1);
   const float d2 = fmaxf(dsq, p1.w);
@@ -290,7 +307,12 @@ template <int S, int K, int MODE, bool ONE, bool CHUNKED>
 __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kernel(const __grid_constant__ KParams p) {
   constexpr int P = 32 / S;      // poses per warp
   constexpr int NB = S * K;      // bead slots per pose
-  constexpr int U = K == 1 ? 1 : 2;  // pair slots in flight per lane
+  // pair slots in flight per lane.  (Builds of K > 1 kernels with small edits, two or four pairs in flight, have
+  // reported misaligned or illegal addresses whose cause is not known: reading, a CPU emulation and
+  // the checked build found every address right.  The K > 1 kernels held here, MODE_MIN's and
+  // MODE_QUAT's, share their source; each of them runs in the tests, guarded and as built, so an edit
+  // here or another compiler has to pass those first.)
+  constexpr int U = K == 1 ? 1 : 2;
   constexpr int PB = pairs_per_bead(K) * NB;  // pair-buffer window of one team
   constexpr bool MAT = (MODE == MODE_EVAL_MAT);
   constexpr bool QUAT = (MODE == MODE_QUAT);   // quaternion + adabelief SCHEMA protocol
@@ -371,6 +393,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 
   while (tile < p.n_tiles) {
     const int si = find_segment(p, tile);
+    if (!ATT_CHECK(si >= 0 && si < p.n_segs && tile >= 0, 13, si, p.n_segs)) break;
     AttSegment sg = p.segs[si];
     // Caller-provided tables are checked before any access they index: the
     // segment's grid, ligand and pose range, the pose's conformer index and
@@ -391,6 +414,10 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
     if (!seg_ok) sg.grid = sg.lig = sg.pose0 = sg.step0 = 0;
     const int b = sg.pose0 + (valid ? local : 0);
     const KGrid& G = ONE ? p.grid[0] : s_grid[ONE ? 0 : sg.grid];
+    if (!ATT_CHECK((((uintptr_t)G.bricks & 127u) | ((uintptr_t)G.nb_rec & 15u) | ((uintptr_t)G.rec & 15u) |
+                    ((uintptr_t)G.pair & 31u)) == 0u, 14, (long long)(uintptr_t)G.pair, (long long)(uintptr_t)G.rec) ||
+        !ATT_CHECK(b >= 0 && (b < p.n_pose_rows || !valid), 15, b, p.n_pose_rows))
+      break;
     int lig = sg.lig;
     if (p.pose_lig != nullptr && valid) {
       lig += __ldg(p.pose_lig + b);
@@ -421,7 +448,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const int i = c0 + tl + k * S;
-        if (i < Ntot) {
+        if (i < Ntot && ATT_CHECK((long long)loff + i < p.n_lig_beads, 16, loff + i, p.n_lig_beads)) {
           const float4 bd = ldg_f4(p.lig_beads + loff + i);
           lx[k] = bd.x; ly[k] = bd.y; lz[k] = bd.z;
           ltw[k] = __float_as_int(bd.w);
@@ -769,11 +796,11 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
           const unsigned sk = (unsigned)(tbase + tl + k * S);
           const unsigned mb = __ballot_sync(0xffffffffu, need_b[k]);
           const unsigned mv = __ballot_sync(0xffffffffu, need_v[k]);
-          if (need_b[k]) {
+          if (need_b[k] && ATT_CHECK(nb_cp + __popc(mb & lanemask_lt()) < 32u * K, 17, nb_cp, 32 * K)) {
             list_b[nb_cp + __popc(mb & lanemask_lt())] = make_uint2((unsigned)bidx[k], sk);
             held_b[k] = bidx[k];
           }
-          if (need_v[k]) {
+          if (need_v[k] && ATT_CHECK(nv_cp + __popc(mv & lanemask_lt()) < 32u * K, 18, nv_cp, 32 * K)) {
             list_v[nv_cp + __popc(mv & lanemask_lt())] = make_uint2((unsigned)nvox[k], sk);
             held_v[k] = nvox[k];
           }
@@ -976,7 +1003,7 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
                   uint32_t* dst = pb + (r + c);
 #pragma unroll
                   for (unsigned i = 0; i < 8; ++i)
-                    if (c + i < nin) dst[i] = v[i];
+                    if (c + i < nin && ATT_CHECK(r + c + i < (unsigned)PB, 19, r + c + i, PB)) dst[i] = v[i];
                 } else {
 #pragma unroll
                   for (unsigned i = 0; i < 8; ++i) {
@@ -1004,7 +1031,9 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
                   continue;
                 }
 #endif
-                for (unsigned s = lo; s < hi; ++s) pb[s - q0] = ldg_nc_u16(G.nb_list + (ovf + (s - r - ninl))) | tag;
+                for (unsigned s = lo; s < hi; ++s)
+                  if (ATT_CHECK(s - q0 < (unsigned)PB, 20, s - q0, PB))
+                    pb[s - q0] = ldg_nc_u16(G.nb_list + (ovf + (s - r - ninl))) | tag;
               }
               r += ck[k];
             }
@@ -1037,7 +1066,8 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
             }
 #pragma unroll
             for (int m = 0; m < U; ++m) {
-              const unsigned bi = tbase + (ww[m] >> 16);
+              unsigned bi = tbase + (ww[m] >> 16);
+              if (!ATT_CHECK(bi < 32u * K, 21, bi, 32 * K)) bi = tbase;
               const BeadPos bp = bpos[bi];
               float px, py, pz;
               pair_term_masked<NE, REF>(p, G, bp, rr[m], jok[m], acc_e, px, py, pz);
