@@ -82,23 +82,91 @@ static cudaError_t launch_one(const KParams& p, int mode, int S, int K, bool one
   return cudaLaunchKernel(k, dim3(blocks), dim3(threads), args, smem, st);
 }
 
+// The launches of one call, one per grid, side by side: each skips the other grids'
+// segments and takes its tiles statically, so that blocks without a tile of its grid end at once.
+// One after another each would end with a tail of its own.  Up to SIDE_STREAMS streams made for
+// the call, between two events of the caller's stream, take the grids in turn with it (to make and
+// destroy one costs the host 110 us; nothing of them outlives the call).  In a stream that is
+// being captured the launches become branches of the graph.  50 steps of 40 beads, one after
+// another and now, against the reference mode's one launch: 2 grids x 500 poses 0.38 -> 0.31 ms
+// (0.23), 8 x 500 1.58 -> 0.72 (0.54; 1, 2 and 7 side streams 0.92, 0.80 and 0.87), 4 x 4000 1.81 -> 1.67
+// (1.62), 8 x 4000 3.64 -> 3.23 (3.10), 8 x 20 000 14.75 -> 14.90 (14.56).
+constexpr int SIDE_STREAMS = 3;
+static cudaError_t launch_side_by_side(const KParams& p, int mode, int S, int K, int blocks, int threads,
+                                       cudaStream_t st) {
+  constexpr size_t MAX_DEPS = 64;
+  KParams q = p;
+  q.counter = nullptr;
+  auto launch = [&](int g, cudaStream_t s) {
+    q.grid[0] = p.grid[g];
+    q.grid_sel = g;
+    return launch_one(q, mode, S, K, true, blocks, threads, s);
+  };
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t n_deps = 0;
+  cudaError_t e = cudaStreamGetCaptureInfo_v2(st, &capture, nullptr, nullptr, &deps, &n_deps);
+  if (e != cudaSuccess) return e;
+
+  if (capture == cudaStreamCaptureStatusActive) {
+    cudaGraphNode_t start[MAX_DEPS], ends[MAX_DEPS];
+    const size_t n_start = n_deps;
+    const bool branches = n_deps <= MAX_DEPS;  // (else one after another)
+    for (size_t i = 0; branches && i < n_start; ++i) start[i] = deps[i];
+    size_t n_ends = 0;
+    for (int g = 0; g < p.n_grids; ++g) {
+      if (branches && g > 0) {
+        e = cudaStreamUpdateCaptureDependencies(st, start, n_start, cudaStreamSetCaptureDependencies);
+        if (e != cudaSuccess) return e;
+      }
+      e = launch(g, st);
+      if (e != cudaSuccess) return e;
+      if (branches) {  // the branch's node
+        e = cudaStreamGetCaptureInfo_v2(st, &capture, nullptr, nullptr, &deps, &n_deps);
+        if (e != cudaSuccess) return e;
+        for (size_t i = 0; i < n_deps && n_ends < MAX_DEPS; ++i) ends[n_ends++] = deps[i];
+      }
+    }
+    return branches ? cudaStreamUpdateCaptureDependencies(st, ends, n_ends, cudaStreamSetCaptureDependencies)
+                    : cudaSuccess;
+  }
+
+  cudaStream_t side[SIDE_STREAMS] = {};
+  cudaEvent_t event = nullptr;
+  int priority = 0, n_side = 0;
+  e = cudaStreamGetPriority(st, &priority);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&event, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventRecord(event, st);
+  for (int g = 0; g < p.n_grids && e == cudaSuccess; ++g) {
+    const int lane = g % (SIDE_STREAMS + 1);  // 0: the caller's stream
+    if (lane == n_side + 1) {
+      if (cudaStreamCreateWithPriority(&side[n_side], cudaStreamNonBlocking, priority) == cudaSuccess) {
+        e = cudaStreamWaitEvent(side[n_side], event, 0);
+        ++n_side;
+      } else {
+        cudaGetLastError();  // none to be had: behind the others
+      }
+    }
+    if (e == cudaSuccess) e = launch(g, lane > 0 && lane <= n_side ? side[lane - 1] : st);
+  }
+  for (int i = 0; i < n_side; ++i) {  // the caller's stream waits for them, whatever became of a launch
+    const cudaError_t e1 = cudaEventRecord(event, side[i]), e2 = cudaStreamWaitEvent(st, event, 0);
+    if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : e2;
+  }
+  for (int i = 0; i < n_side; ++i) cudaStreamDestroy(side[i]);  // (freed when its work is done)
+  if (event != nullptr) cudaEventDestroy(event);
+  return e;
+}
+
 // One launch, but for the analytic gradient of a minimiser over several grids with
-// several beads per lane: one per grid over the same tiles, each skipping the other grids'
-// segments.  (Those kernels hold the reference mode only.  Compiled with both, a
-// 32-lane, two-beads-per-lane evaluation over two grids reported a misaligned address in
-// the analytic mode, where the bounds-checked build of the same source found
-// every index and alignment right.)
+// several beads per lane: one per grid over the same tiles.  (Those kernels hold the
+// reference mode only.  Compiled with both, a 32-lane, two-beads-per-lane evaluation over
+// two grids reported a misaligned address in the analytic mode, where the bounds-checked
+// build of the same source found every index and alignment right.)
 cudaError_t launch_score(const KParams& p, int mode, int S, int K, int blocks, int threads, cudaStream_t st) {
   if (p.n_grids == 1 || K == 1 || p.grad_mode == ATT_GRAD_REFERENCE)
     return launch_one(p, mode, S, K, p.n_grids == 1, blocks, threads, st);
-  KParams q = p;
-  for (int g = 0; g < p.n_grids; ++g) {
-    q.grid[0] = p.grid[g];
-    q.grid_sel = g;
-    const cudaError_t e = launch_one(q, mode, S, K, true, blocks, threads, st);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  return launch_side_by_side(p, mode, S, K, blocks, threads, st);
 }
 
 // the bits of every part's error word
