@@ -643,11 +643,14 @@ cudaError_t launch_nb_quantile(const uint32_t* hdr, long long nvox, float q, lon
   unsigned long long* total = reinterpret_cast<unsigned long long*>(words + (nblk + 3) / 2 * 2);
   unsigned* hist = reinterpret_cast<unsigned*>((reinterpret_cast<uintptr_t>(total + 1) + 15) & ~(uintptr_t)15);
   const uint2* h = reinterpret_cast<const uint2*>(hdr);
-  cudaError_t e = cudaMemsetAsync(hist, 0, HIST_BINS * sizeof(unsigned), st);
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, HIST_BINS * sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
   nb_nonzero_kernel<<<nblk, HIST_THREADS, 0, st>>>(h, nvox, words);
   nb_scan_blocks_kernel<<<1, SCAN_THREADS, 0, st>>>(words, nblk, total);
-  nb_hist_kernel<<<min(nblk, 148 * 8), HIST_THREADS, 0, st>>>(h, nvox, words, nblk, first, hist);
+  nb_hist_kernel<<<min(nblk, sms * 8), HIST_THREADS, 0, st>>>(h, nvox, words, nblk, first, hist);
   nb_quantile_kernel<<<1, SCAN_THREADS, 0, st>>>(hist, total, first, q, out);
   return cudaGetLastError();
 }

@@ -82,18 +82,6 @@ struct KParams {
 
 __device__ __forceinline__ float4 ldg_f4(const float4* p) { return __ldg(p); }
 
-// Grid bricks are streamed: keep them out of L1 so that the receptor, pair
-// table and ligand beads stay resident there.
-__device__ __forceinline__ float4 ldg_stream_f4(const float4* p) {
-  float4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "l"(p));
-  return v;
-}
-
-__device__ __forceinline__ uint2 ldg_u2(const uint2* p) { return __ldg(p); }
-
 // One 32-byte row (two float4) in a single 256-bit read-only load: a gather
 // of such rows touches each cache line once per instruction instead of twice.
 // p must be 32-B aligned.
