@@ -339,6 +339,10 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
   // sums cost a warp 1 % of 301 beads, 3 % of 100; two chunks are summed as one class.)
   constexpr bool CLASSES = CHUNKED && MODE != MODE_MIN && !QUAT;
   const bool split = CLASSES && p.split != 0;
+  // A pose of one or two chunks beside larger ones of its warp (conformers of different
+  // sizes in one segment) still sums them as one class: it takes its second chunk in the first
+  // class's second step.
+  constexpr bool MIXED = CLASSES && S < 32;
   // the pair loop and phase D are compiled per gradient mode; with several beads
   // per lane the kernels over several grids hold the reference mode only (launch_score)
   const bool ref_grad = (!ONE && K > 1) || p.grad_mode == ATT_GRAD_REFERENCE;
@@ -609,10 +613,13 @@ __global__ void __launch_bounds__(128, (score_blocks_per_sm<S, K>())) score_kern
 #pragma unroll
       for (int k = 0; k < (CLASSES && !SCATTER ? NS : 1); ++k) all_tot[k] = 0.f;
       const bool classes = CLASSES && nchunk > 2;
+      const bool one_class = MIXED && classes && Ntot <= 2 * NB;
+      const bool any_second = MIXED && __any_sync(0xffffffffu, one_class && Ntot > NB);
       const int cls_end = classes ? min(nchunk, 4) : 1;
       for (int cls = split ? warp : 0; cls < cls_end; cls += split ? 4 : 1) {
-      for (int chunk = cls; chunk < (CHUNKED ? nchunk : 1); chunk += classes ? 4 : 1) {
-      const int c0 = chunk * NB;
+      const int chunk_end = MIXED && any_second && cls == 0 ? max(nchunk, 5) : nchunk;
+      for (int chunk = cls; chunk < (CHUNKED ? chunk_end : 1); chunk += classes ? 4 : 1) {
+      const int c0 = (one_class ? cls == 0 ? chunk >> 2 : nchunk : chunk) * NB;
       const int N = max(0, min(Ntot - c0, NB));  // beads of this chunk
       if (multi) load_beads(c0);
       // ---------------- phase A: move beads, start brick copies, list headers
