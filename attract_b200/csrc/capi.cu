@@ -210,7 +210,9 @@ static int fill_common(KParams* p, int mode, const AttGrid* grids, int n_grids, 
   p->rec_slot = rec_slot;
   REQUIRE(!launch || launch->test_flags == 0, "AttLaunchCfg.test_flags is reserved and must be 0");
   p->test_flags = 0;
-  if (launch && launch->block_threads) {  // a caller's block has to hold whole ligands
+  if (launch && launch->block_threads) {
+    // a caller's block has to hold whole ligands, also in the single evaluations, whose kernels
+    // need one bead per lane only: what was refused before they did stays refused
     REQUIRE(score_smem_bytes(all, t, rec_slot) <= kDynSmemLimit,
             "%d threads x %d beads per lane need %zu B of shared memory", t, all, score_smem_bytes(all, t, rec_slot));
   } else {  // default: the largest block whose shared memory fits

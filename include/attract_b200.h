@@ -64,9 +64,16 @@ extern "C" {
                                    pose's conformer index (pose_lig) or its ligand's bead range left the ligand
                                    set: those poses were skipped (outputs unwritten), checked before any access */
 
-/* A pose is served by lanes_per_pose lanes holding up to 8 beads each; a
-   ligand with more than 8 * lanes_per_pose beads is evaluated in chunks of that
-   many beads (slower: its coordinates are re-read every chunk). */
+/* In a minimisation (att_minimise, att_minimise_schema) the lanes_per_pose lanes
+   of a pose hold up to 8 beads each; a ligand with more than 8 * lanes_per_pose
+   beads is evaluated in chunks of that many beads (slower: its coordinates are
+   re-read every chunk).  In a single evaluation (att_energrad,
+   att_energrad_backward) a lane holds one bead and a chunk is lanes_per_pose beads;
+   from three chunks on they are summed in four classes (chunk mod 4), whatever
+   the poses beside it.
+   The minimisers' kernels with several beads per lane share their source with
+   builds that reported memory faults of unknown cause (csrc/score.cu, at U): an edit of
+   them or another compiler has to pass the checked build's tests first. */
 #define ATT_MAX_BEADS_PER_LANE 8
 
 /* Geometry of one receptor grid: the scalar fields of read_grid2.py's Grid. */
@@ -170,7 +177,8 @@ typedef struct AttSchemaCfg {
 /* Launch shape; zeros pick the defaults / autotuned values. */
 typedef struct AttLaunchCfg {
   int lanes_per_pose;   /* 8, 16 or 32 (poses per warp = 32 / lanes_per_pose) */
-  int block_threads;    /* 32, 64, 96 or 128 (0 = the largest whose shared memory fits) */
+  int block_threads;    /* 32, 64, 96 or 128 (0 = the largest whose shared memory fits); a given size
+                           has to hold whole ligands at up to 8 beads per lane, in every call */
   int blocks;           /* persistent CTAs (att_minimise), 0 = fill the GPU */
   int test_flags;       /* reserved: must be 0 */
 } AttLaunchCfg;
