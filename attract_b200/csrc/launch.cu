@@ -1,5 +1,7 @@
 // Launches of the scoring kernels (score.cu): the kernel of a launch, its
 // shared memory and occupancy, and the kernels' error words.
+#include <mutex>
+
 #include "score_parts.h"
 
 namespace att {
@@ -82,15 +84,76 @@ static cudaError_t launch_one(const KParams& p, int mode, int S, int K, bool one
   return cudaLaunchKernel(k, dim3(blocks), dim3(threads), args, smem, st);
 }
 
+// Side streams of launch_side_by_side.  To make and destroy one costs the host 110 us, so up to
+// KEPT of them stay for later calls (in any thread).  A call takes one only when its work is done and makes
+// another otherwise: no caller's stream ever waits for another's.  They belong to a context; its id is never
+// used twice, so streams of one that was reset are not touched again.
+struct SideStream {
+  cudaStream_t stream;
+  unsigned long long ctx;
+  int priority;
+};
+struct SideStreams {
+  static constexpr int KEPT = 8;
+  std::mutex mutex;
+  SideStream kept[KEPT];
+  int n = 0;
+};
+static SideStreams g_side_streams;  // (for the process: no CUDA call at its exit)
+
+static unsigned long long context_id() {  // 0: not to be had
+  typedef int (*CtxGetId)(void*, unsigned long long*);
+  static const CtxGetId fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<CtxGetId>(f);
+  }();
+  unsigned long long id = 0;
+  return fn != nullptr && fn(nullptr, &id) == 0 ? id : 0;
+}
+
+static cudaError_t take_side_stream(unsigned long long ctx, int priority, cudaStream_t* out) {
+  if (ctx != 0) {
+    SideStreams& s = g_side_streams;
+    std::lock_guard<std::mutex> lock(s.mutex);
+    for (int i = 0; i < s.n; ++i)
+      if (s.kept[i].ctx == ctx && s.kept[i].priority == priority) {
+        const cudaError_t e = cudaStreamQuery(s.kept[i].stream);
+        if (e == cudaErrorNotReady) {
+          cudaGetLastError();
+        } else {
+          *out = s.kept[i].stream;
+          s.kept[i] = s.kept[--s.n];
+          return e;
+        }
+      }
+  }
+  return cudaStreamCreateWithPriority(out, cudaStreamNonBlocking, priority);
+}
+static void give_side_stream(unsigned long long ctx, int priority, cudaStream_t stream) {
+  if (ctx != 0) {
+    SideStreams& s = g_side_streams;
+    std::lock_guard<std::mutex> lock(s.mutex);
+    if (s.n < SideStreams::KEPT) {
+      s.kept[s.n++] = {stream, ctx, priority};
+      return;
+    }
+  }
+  cudaStreamDestroy(stream);  // (freed when its work is done)
+}
+
 // The launches of one call, one per grid, side by side: each skips the other grids'
 // segments and takes its tiles statically, so that blocks without a tile of its grid end at once.
-// One after another each would end with a tail of its own.  Up to SIDE_STREAMS streams made for
-// the call, between two events of the caller's stream, take the grids in turn with it (to make and
-// destroy one costs the host 110 us; nothing of them outlives the call).  In a stream that is
+// One after another each would end with a tail of its own.  Up to SIDE_STREAMS side streams,
+// between two events of the caller's stream, take the grids in turn with it.  In a stream that is
 // being captured the launches become branches of the graph.  50 steps of 40 beads, one after
-// another and now, against the reference mode's one launch: 2 grids x 500 poses 0.38 -> 0.31 ms
-// (0.23), 8 x 500 1.58 -> 0.72 (0.54; 1, 2 and 7 side streams 0.92, 0.80 and 0.87), 4 x 4000 1.81 -> 1.67
-// (1.62), 8 x 4000 3.64 -> 3.23 (3.10), 8 x 20 000 14.75 -> 14.90 (14.56).
+// another and now: 2 grids x 500 poses 0.56 -> 0.29 ms, 8 x 500 2.41 -> 0.70, 4 x 4000 2.37 -> 2.05, 8 x 4000
+// 4.75 -> 3.94; 1 step of 4 poses on each of 8 grids 0.18 -> 0.06 (0.35 with streams made for the call).
+// (On an easier case 8 x 500 took 1.58 -> 0.72, 0.54 in the reference mode's one launch; 1, 2 and 7 side
+// streams 0.92, 0.80 and 0.87.)
 constexpr int SIDE_STREAMS = 3;
 static cudaError_t launch_side_by_side(const KParams& p, int mode, int S, int K, int blocks, int threads,
                                        cudaStream_t st) {
@@ -134,13 +197,18 @@ static cudaError_t launch_side_by_side(const KParams& p, int mode, int S, int K,
   cudaStream_t side[SIDE_STREAMS] = {};
   cudaEvent_t event = nullptr;
   int priority = 0, n_side = 0;
+  const unsigned long long ctx = context_id();
+  // (another thread may be capturing: nothing here touches its stream)
+  cudaStreamCaptureMode mode_before = cudaStreamCaptureModeRelaxed;
+  e = cudaThreadExchangeStreamCaptureMode(&mode_before);
+  if (e != cudaSuccess) return e;
   e = cudaStreamGetPriority(st, &priority);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&event, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventRecord(event, st);
   for (int g = 0; g < p.n_grids && e == cudaSuccess; ++g) {
     const int lane = g % (SIDE_STREAMS + 1);  // 0: the caller's stream
     if (lane == n_side + 1) {
-      if (cudaStreamCreateWithPriority(&side[n_side], cudaStreamNonBlocking, priority) == cudaSuccess) {
+      if (take_side_stream(ctx, priority, &side[n_side]) == cudaSuccess) {
         e = cudaStreamWaitEvent(side[n_side], event, 0);
         ++n_side;
       } else {
@@ -153,8 +221,9 @@ static cudaError_t launch_side_by_side(const KParams& p, int mode, int S, int K,
     const cudaError_t e1 = cudaEventRecord(event, side[i]), e2 = cudaStreamWaitEvent(st, event, 0);
     if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : e2;
   }
-  for (int i = 0; i < n_side; ++i) cudaStreamDestroy(side[i]);  // (freed when its work is done)
+  for (int i = 0; i < n_side; ++i) give_side_stream(ctx, priority, side[i]);
   if (event != nullptr) cudaEventDestroy(event);
+  cudaThreadExchangeStreamCaptureMode(&mode_before);
   return e;
 }
 
@@ -166,6 +235,20 @@ static cudaError_t launch_side_by_side(const KParams& p, int mode, int S, int K,
 cudaError_t launch_score(const KParams& p, int mode, int S, int K, int blocks, int threads, cudaStream_t st) {
   if (p.n_grids == 1 || K == 1 || p.grad_mode == ATT_GRAD_REFERENCE)
     return launch_one(p, mode, S, K, p.n_grids == 1, blocks, threads, st);
+  // Many tiles: one after another, tiles from the counter.  Static tiles end about a wave unevenly,
+  // each tail saved is worth part of one: even at 3 waves of a grid for 2 grids, 6 to 8 for 4 (50 steps of 40 beads:
+  // 2 x 6000 poses 1.61 -> 1.65 ms, 2 x 20 000 4.52 -> 4.70, 4 x 10 000 4.96 -> 4.80, 4 x 20 000 9.10 -> 9.19, 8 x 10 000
+  // 10.03 -> 9.36; a wave is 2368 poses here).
+  if (2LL * p.n_tiles > 3LL * p.n_grids * p.n_grids * blocks * (threads / 32)) {
+    KParams q = p;
+    cudaError_t e = cudaSuccess;
+    for (int g = 0; g < p.n_grids && e == cudaSuccess; ++g) {
+      q.grid[0] = p.grid[g];
+      q.grid_sel = g;
+      e = launch_one(q, mode, S, K, true, blocks, threads, st);
+    }
+    return e;
+  }
   return launch_side_by_side(p, mode, S, K, blocks, threads, st);
 }
 
