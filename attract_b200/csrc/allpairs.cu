@@ -13,10 +13,10 @@
 // with whole receptors, a handful of poses needs every split there is.
 //
 // A pose's results do not depend on the split, nor on the poses beside it.  The
-// receptor is divided into leaves (a power of two, 33 to 64 beads each) that
+// receptor is divided into leaves (a power of two, 17 to 64 beads each) that
 // follow from its length alone.  A lane sums an item's energy and force over a
-// leaf in float, then in double: the four leaves of a branch in order (more of them
-// beyond 16 384 beads), the branches in a binary tree, whose lower levels a
+// leaf in float, then in double: the leaves of a branch in order (four; two or
+// more of 64 branches beyond 4096 beads), the branches in a binary tree, whose lower levels a
 // lane forms by itself and whose upper ones the groups and the cluster's blocks.
 // A pose's sum takes its beads 64 at a time.
 //
@@ -26,8 +26,8 @@
 // receptor beads at once (a row test and shuffles of its own per bead).  2500 x
 // 24 beads: 16 384 poses 1958 -> 880 us (1.1 T pairs/s), 10 poses 48 us on one block each -> 13.4,
 // below the host's part of the call.  (Splits chosen without regard to the sums' order took
-// 889 and 12.9 us; 300 poses 31 us against 41, 5000 x 24 beads, 10 poses 16 against 30, 5000 x
-// 301 beads, 300 poses 609 against 504.)
+// 889 and 12.9 us; 300 poses 31 us against 41, 150 x 24 beads, 16 384 poses 135 against 145, 5000 x 24
+// beads, 10 poses 16 against 21, 5000 x 301 beads, 300 poses 609 against 511.)
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -143,15 +143,18 @@ __device__ __forceinline__ PoseM load_pose(const AllPairsParams& p, int b) {
   return q;
 }
 
-// The receptor's leaves, the smallest power of two that leaves each 64 beads or fewer, and its
-// branches.  (Leaves as branches cost 2500 x 24 beads, 16 384 poses 1 %, 300 x 8 beads 4 %.)
+// The receptor's leaves, the smallest power of two that leaves each 32 beads or fewer, from 64
+// leaves on 64 beads, and its branches.  A leaf is the shortest piece that few poses can be split into: with 64
+// beads throughout 10 poses of 24 beads took 15.8 us on 150 beads (now 11.5), 14.8 on 700 (11.9), and
+// 16 384 poses 137 (now 145) and 310 (332).  (Leaves as branches: 2500 x 24 beads, 16 384 poses 1 %,
+// 300 x 8 beads 4 % slower.)
 static int ap_leaves_log2(int n_rec) {
   int n = 0;
-  while (((long long)AP_LEAF << n) < n_rec) ++n;
+  while (((long long)(n < 6 ? AP_LEAF / 2 : AP_LEAF) << n) < n_rec) ++n;
   return n;
 }
 static int ap_branches_log2(int leaves_log2) {
-  return leaves_log2 < 2 ? 0 : leaves_log2 - 2 < AP_LEVELS ? leaves_log2 - 2 : AP_LEVELS;
+  return leaves_log2 > 6 ? AP_LEVELS : leaves_log2 > 2 ? leaves_log2 - 2 : 0;
 }
 
 constexpr int ap_slots(int NP) { return AP_WARPS * 64 * NP; }  // items of a block, over its receptor groups
@@ -554,8 +557,8 @@ static ApKernel ap_kernel(bool cut, bool grad) {
 // without a block).  A block alone on an SM takes its steps (a receptor bead against a lane's
 // items; 1.2 at two packed pairs), 20 steps per pass over the ligand, 20 for its start and
 // sums and 2.7 per block of its cluster; each further block of busy warps adds 0.2 (0.435)
-// of a step to a step.  Fitted to all splits of 60 calls of 150-17 000 receptor beads, 8-301 ligand beads
-// and 10-40 000 poses: the split taken is within 2 % of the fastest on average (100 poses of 130 beads: 23 %),
+// of a step to a step.  Fitted to all splits of 75 calls of 60-17 000 receptor beads, 8-301 ligand beads
+// and 1-60 000 poses: the split taken is within 3 % of the fastest on average (10 poses of 301 beads: 26 %),
 // where the slowest is 3 to 10 times slower.
 struct ApPlan {
   int np, rw, cl, pb, nb;

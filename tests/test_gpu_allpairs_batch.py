@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
     (1, 1, 0.0, False), (64, 3, 0.0, True), (65, 24, 0.0, False), (130, 64, 9.0, True), (700, 65, 0.0, True),
     (2047, 7, 0.0, False), (2049, 130, 0.0, True), (2500, 24, 0.0, False), (2500, 24, 15.0, True), (5000, 24, 0.0, True),
     (300, 1100, 0.0, False),
-    (17000, 3, 0.0, True)])
+    (17000, 3, 0.0, True), (33, 24, 0.0, True), (150, 24, 0.0, False), (4097, 10, 0.0, False)])
 def test_a_pose_alone_and_in_a_library(n_rec, beads, rcut, mix):
     import attract_b200 as A
     from attract_b200.allpairs import AllPairs
